@@ -124,7 +124,7 @@ def workload(name, steps, seed=2024):
                                '1.4 outside a 6x6x3 um Si block), CPML 12, Yee sampling, Ey dipole, FP32')
     if name in ('tfsf', 'dispersive'):
         # 256^3 at 0.05 um, CPML 12: a TFSF box (plane wave along +x) around a Si sphere, or a Drude sphere and a
-        # Lorentz slab lit by an Ey dipole; both run the split gather step.
+        # Lorentz slab lit by an Ey dipole; both run the two-pass step.
         n, L = (256, 256, 256), 12
         b = Boundaries(**{f'{a}_{s}': baseline_face(L) for a in 'xyz' for s in ('min', 'max')})
         region = Region(dimension='3d', size=tuple(v * .05 for v in n), mesh=.05, pml_cells=L, steps=steps, backend='cuda',

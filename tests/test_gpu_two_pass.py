@@ -1,0 +1,93 @@
+"""The two-pass step kernels against the NumPy oracle: every way they are launched (three launches per step, one cluster,
+one cooperative launch), at row lengths around the 16-byte groups, and with more than two CPML slabs on an axis (the
+row-table path). Bar: fields, CPML memories and traces bitwise, like the other step kernels (same operations, same
+order, no contraction)."""
+from dataclasses import replace
+
+import numpy as np
+import pytest
+
+from oracle.yee_oracle import YeeOracle
+from torchfdtd_b200 import Project, Region
+from torchfdtd_b200.models import BoundaryFace, Monitor, Source
+from torchfdtd_b200.plan import plan_grid
+
+pytestmark = pytest.mark.gpu
+
+
+def scene(shape, precision, faces=None, component='Ey', steps=12):
+    two_d = shape[2] == 1
+    region = Region(dimension='2d' if two_d else '3d', size=tuple(n * .05 for n in shape[:2]) + (1 if two_d else shape[2] * .05,),
+                    mesh=.05, pml_cells=4, steps=steps, precision=precision, backend='cuda')
+    for name, face in (faces or {}).items():
+        setattr(region.boundaries, name, face)
+    return Project(region=region, sources=[Source(center=(.1, 0, 0), component=component, pulse_cycles=1, wavelength=.6)],
+                   monitors=[Monitor(center=(-.1, .05, 0), component=component)])
+
+
+def assert_matches_oracle(plan, seed, kernel='gather'):
+    from torchfdtd_b200.native import NativeGrid
+    rng = np.random.default_rng(seed)
+    oracle = YeeOracle(plan)
+    advanced = plan.active_components()
+    for family, field in (('E', oracle.E), ('H', oracle.H)):
+        for c in range(3):
+            if family + 'xyz'[c] in advanced:
+                field[..., c] = rng.normal(size=plan.shape).astype(plan.dtype)
+    grid = NativeGrid(plan, kernel=kernel)
+    grid.set_fields(oracle.E, oracle.H)
+    grid.step(5)
+    grid.step(plan.steps - 5)
+    oracle.run()
+    E, H = grid.get_fields()
+    np.testing.assert_array_equal(E, oracle.E)
+    np.testing.assert_array_equal(H, oracle.H)
+    np.testing.assert_array_equal(grid.get_traces(), oracle.traces)
+    for got, want in zip(grid.get_psi(), oracle.memory_states):
+        np.testing.assert_array_equal(got, want)
+    assert grid.counter() == plan.steps and grid.device_status() == 0
+    grid.close()
+
+
+PERIODIC_Y = {'y_min': BoundaryFace(kind='periodic'), 'y_max': BoundaryFace(kind='periodic')}
+
+
+@pytest.mark.parametrize('mode', ['0', '1', '2'])
+@pytest.mark.parametrize('shape,precision,faces,component', [
+    ((13, 14, 15), 'float32', None, 'Ey'), ((14, 13, 16), 'float64', {'z_max': BoundaryFace(kind='pec')}, 'Hz'),
+    ((32, 13, 14), 'float32', PERIODIC_Y, 'Ez'), ((65, 33, 1), 'float32', PERIODIC_Y, 'Hz'), ((67, 40, 1), 'float64', None, 'Ex')])
+def test_every_launch_form_matches_the_oracle(monkeypatch, mode, shape, precision, faces, component):
+    monkeypatch.setenv('TFD_PASS_STEPS', mode)
+    assert_matches_oracle(plan_grid(scene(shape, precision, faces, component)), 3)
+
+
+@pytest.mark.parametrize('precision', ['float32', 'float64'])
+def test_more_than_two_slabs_on_an_axis(precision):
+    plan = plan_grid(scene((21, 18, 16), precision))
+    segments = []                                       # x slabs in two parts each; no z slabs (12 segments at most)
+    for s in plan.segments:
+        cut = (s.lo + s.hi) // 2 if s.axis == 0 else s.hi
+        for lo, hi in ((s.lo, cut), (cut, s.hi)):
+            if lo < hi and s.axis < 2:
+                part = slice(lo - s.lo, hi - s.lo)
+                segments.append(replace(s, lo=lo, hi=hi, b=s.b[part], c=s.c[part], inv_kappa=s.inv_kappa[part]))
+    assert len(segments) == 12
+    assert_matches_oracle(replace(plan, segments=segments), 4)
+
+
+@pytest.mark.parametrize('shape,steps', [((40, 30, 20), 3), ((24, 22, 260), 2)])
+def test_default_3d_step_equals_the_marching_kernel(shape, steps):
+    from torchfdtd_b200.native import NativeGrid
+    plan = plan_grid(scene(shape, 'float32', steps=10))
+    rng = np.random.default_rng(1)
+    start = [rng.normal(size=(*plan.shape, 3)).astype(np.float32) for _ in range(2)]
+    out = []
+    for variant in (0, 14):
+        grid = NativeGrid(plan, variant=variant)
+        assert grid.kernel == 'march'
+        grid.set_fields(*start)
+        grid.step(steps)
+        out.append((*grid.get_fields(), *grid.get_psi()))
+        grid.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)

@@ -10,8 +10,8 @@
 #include "aux.cuh"
 #include "internal.cuh"
 #include "persist2d.cuh"
-#include "step_gather.cuh"
 #include "step_march.cuh"
+#include "step_pass.cuh"
 #include "step2d.cuh"
 #include "adjoint.cuh"
 #include "cluster2d.cuh"
@@ -108,7 +108,7 @@ struct Layout {
     size_t ade_map = 0;            // 3 x count int32 sample indices
     size_t volume[3];              // diagnostics cell volumes per axis (double), 0: unit
     size_t counter = 0, done = 0, status = 0, diag = 0, stage = 0;
-    size_t grid_bar = 0;           // persistent 2D stepping: arrival count and generation
+    size_t grid_bar = 0;           // persistent stepping: arrival count and generation
     size_t check = 0;              // tfd_set_permittivity / tfd_field_check results
     size_t grid_tab = 0, tile_tab = 0;   // 2D tile kernel: this plan's Grid struct and its tile table
     int tiles2d = 0, strip_rows = 8;
@@ -478,10 +478,17 @@ struct tfd_plan {
     MarchMix march_mix{};
     std::vector<MarchLaunch> march_launches;
     bool march_metric = false;     // nonuniform mesh: the general body with metric factors
-    TfsfArgs<float> tf{};          // TFSF boxes (the step runs the split gather kernels when there are any)
+    PassArgs<float> pf;            // two-pass step (kernel 'gather')
+    PassArgs<double> pd;
+    bool pass_metric = false, pass_wide = false;
+    int pass_ctas = 0;             // > 0: all steps of a call in one launch of this many CTAs (pass_cluster: one cluster)
+    bool pass_cluster = false;
+    bool two_pass = false;         // the steps run as two passes (kernel 'gather', and 'march' where two_pass_3d says so)
+    template <typename T> PassArgs<T> &pass();
+    TfsfArgs<float> tf{};          // TFSF boxes (corrections land between and after the passes)
     TfsfArgs<double> td{};
     double tfsf_index[kMaxTfsf] = {}, tfsf_norm[kMaxTfsf] = {};   // diagnostics: background index, norm weight
-    bool split = false;            // TFSF boxes or dispersive materials: the split gather step
+    bool split = false;            // TFSF boxes or dispersive materials: the two-pass step only
     // Diagnostics of the dispersive states: per state and pole the divisors of Q and the factors of P.
     std::vector<std::vector<double>> ade_cq, ade_cp;
     template <typename T> TfsfArgs<T> &tfsf();
@@ -513,6 +520,8 @@ template <> Grid<float> &tfd_plan::grid<float>() { return gf; }
 template <> Grid<double> &tfd_plan::grid<double>() { return gd; }
 template <> MarchArgs<float> &tfd_plan::march<float>() { return mf; }
 template <> MarchArgs<double> &tfd_plan::march<double>() { return md; }
+template <> PassArgs<float> &tfd_plan::pass<float>() { return pf; }
+template <> PassArgs<double> &tfd_plan::pass<double>() { return pd; }
 template <> TfsfArgs<float> &tfd_plan::tfsf<float>() { return tf; }
 template <> TfsfArgs<double> &tfd_plan::tfsf<double>() { return td; }
 
@@ -1478,16 +1487,188 @@ MonitorArgs<T> monitor_args(tfd_plan *p) {
 }
 
 template <typename T>
-int launch_step_gather(tfd_plan *p, cudaStream_t s) {
-    const Grid<T> &g = p->grid<T>();
-    dim3 block(128), grid((unsigned)((long long)g.n[1] * g.n[2]), (unsigned)((g.n[0] + 127) / 128));
-    // rows on x (up to 2^31-1), x chunks on y
-    switch (g.active) {
-        case kMaskTM: k_step_gather_rows<T, kMaskTM><<<grid, block, 0, s>>>(g); break;
-        case kMaskTE: k_step_gather_rows<T, kMaskTE><<<grid, block, 0, s>>>(g); break;
-        default: k_step_gather_rows<T, kMaskAll><<<grid, block, 0, s>>>(g); break;
+using PassSteps = void (*)(const PassArgs<T>, const MonitorArgs<T>, int, int, int, unsigned *);
+
+template <typename T, int ACTIVE, bool CLUSTER>
+PassSteps<T> pass_steps_of(bool metric, bool ade) {
+    if (ade) return k_pass_steps<T, ACTIVE, true, true, CLUSTER>;      // (a uniform mesh's factors are 1)
+    return metric ? k_pass_steps<T, ACTIVE, true, false, CLUSTER> : k_pass_steps<T, ACTIVE, false, false, CLUSTER>;
+}
+
+template <typename T>
+PassSteps<T> pass_steps_kernel(tfd_plan *p, bool cluster) {
+    const PassArgs<T> &a = p->pass<T>();
+    const bool ade = a.g.n_ade > 0;
+    switch (a.g.active) {
+        case kMaskTM: return cluster ? pass_steps_of<T, kMaskTM, true>(p->pass_metric, ade) : pass_steps_of<T, kMaskTM, false>(p->pass_metric, ade);
+        case kMaskTE: return cluster ? pass_steps_of<T, kMaskTE, true>(p->pass_metric, ade) : pass_steps_of<T, kMaskTE, false>(p->pass_metric, ade);
+        default: return cluster ? pass_steps_of<T, kMaskAll, true>(p->pass_metric, ade) : pass_steps_of<T, kMaskAll, false>(p->pass_metric, ade);
+    }
+}
+
+constexpr long long kMarchMinCells = 1LL << 26;      // see two_pass_3d
+// Steps in one launch (k_pass_steps): one cluster while a pass is one group per thread of its 16 CTAs (a 200 x 121 TE grid:
+// 7.1 us per step, 9.3 with the grid barrier, 11.0 with three launches per step), the grid barrier up to kPassGridGroups
+// (320 x 240 cells: 8.8 us against 10.7 in the cluster and 10.8; 160 x 120 x 40 cells: 27.0 against 32.0; but 192^3 cells,
+// 1.8 M groups: 147 against 136) or three times that in FP64, where both forms run 512 threads per SM (151 x 133 x 117
+// cells, 1.2 M groups: 91 against 102).
+constexpr int kPassClusterRanks = 16;
+constexpr long long kPassClusterGroups = (long long)kPassClusterRanks * kPassStepThreads, kPassGridGroups = 1LL << 19;
+
+inline void pass_steps_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &attr, bool cluster, int ctas, cudaStream_t s) {
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3(kPassStepThreads);
+    cfg.stream = s;
+    if (cluster) {
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = (unsigned)ctas;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    } else {
+        attr.id = cudaLaunchAttributeCooperative;
+        attr.val.cooperative = 1;
+    }
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+}
+
+// Whether the plan's steps run in one launch, and on how many CTAs.
+template <typename T>
+int setup_pass_steps(tfd_plan *p) {
+    const PassArgs<T> &a = p->pass<T>();
+    p->pass_ctas = 0;
+    const char *env = getenv("TFD_PASS_STEPS");
+    const int mode = env ? std::atoi(env) : -1;
+    if (p->pass_wide || p->desc.n_tfsf > 0 || mode == 0) return TFD_OK;
+    const long long groups = (long long)a.split[0].total * a.g.n[2];
+    const int mblocks = std::max(1, (p->max_samples + kPassStepThreads - 1) / kPassStepThreads) * std::max(1, p->desc.n_planes);
+    if (mode == 1 || (mode < 0 && groups <= kPassClusterGroups)) {
+        PassSteps<T> kernel = pass_steps_kernel<T>(p, true);
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr;
+        pass_steps_config(cfg, attr, true, kPassClusterRanks, nullptr);
+        int clusters = 0;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters >= 1) {
+            p->pass_ctas = kPassClusterRanks;
+            p->pass_cluster = true;
+            return TFD_OK;
+        }
+        cudaGetLastError();
+    }
+    if (mode == 2 || (mode < 0 && groups <= kPassGridGroups * (sizeof(T) == 8 ? 3 : 1))) {
+        int device = 0, sms = 148, per_sm = 0;
+        TFD_CUDA(cudaGetDevice(&device));
+        TFD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+        TFD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass_steps_kernel<T>(p, false), kPassStepThreads, 0));
+        const long long want = std::max<long long>((groups + kPassStepThreads - 1) / kPassStepThreads, mblocks);
+        if (per_sm > 0) p->pass_ctas = (int)std::min<long long>(want, (long long)sms * 1);
+        p->pass_cluster = false;
     }
     return TFD_OK;
+}
+
+template <typename T>
+int launch_pass_steps(tfd_plan *p, int nsteps, cudaStream_t s) {
+    const PassArgs<T> &a = p->pass<T>();
+    const MonitorArgs<T> m = monitor_args<T>(p);
+    const int mgx = std::max(1, (p->max_samples + kPassStepThreads - 1) / kPassStepThreads), mgy = std::max(1, p->desc.n_planes);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr;
+    pass_steps_config(cfg, attr, p->pass_cluster, p->pass_ctas, s);
+    unsigned *bar = p->ptr<unsigned>(p->L.grid_bar);
+    // The barrier word starts every launch at zero: a launch that timed out leaves its arrival count behind.
+    if (!p->pass_cluster) TFD_CUDA(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), s));
+    TFD_CUDA(cudaLaunchKernelEx(&cfg, pass_steps_kernel<T>(p, p->pass_cluster), a, m, mgx, mgy, nsteps, bar));
+    return TFD_OK;
+}
+
+// Whether a 3D plan steps in two passes instead of the marching kernel. The marching kernel moves 52 bytes per cell
+// against 76, but needs the largest grids to get there; measured, us per step (two-pass / march): 160 x 120 x 40: 27 /
+// 43; 192^3: 136 / 207; 256^3: 281 / 398; 320^3: 514 / 647; 400^3: 971 / 1018; 512 x 512 x 256: 960-990 / 907. With
+// periodic x / y faces (512 x 512 x 128: 465 / 626), a nonuniform mesh (306 x 306 x 176: 314 / 379) or in FP64 (151 x 133 x
+// 117, periodic: 89 / 222) the marching kernel runs slower bodies and the two passes win at every size tried. An
+// explicit launch variant (or TFD_MARCH_VARIANT) asks for the marching kernel.
+bool two_pass_3d(const tfd_plan *p) {
+    const tfd_desc &d = p->desc;
+    if (d.launch_variant != 0 || getenv("TFD_MARCH_VARIANT")) return false;
+    const bool seams = d.face[0][0] == TFD_FACE_PERIODIC || d.face[1][0] == TFD_FACE_PERIODIC;
+    return d.precision == 8 || p->march_metric || seams || (long long)d.nx * d.ny * d.nz < kMarchMinCells;
+}
+
+// The two-pass step's arguments: the grid, its slab bounds (or, with more than two slabs on an axis, the row
+// tables) and the 16-byte groups of a row.
+template <typename T>
+int setup_pass(tfd_plan *p) {
+    PassArgs<T> &a = p->pass<T>();
+    std::memset(&a, 0, sizeof(a));
+    a.g = p->grid<T>();
+    int count[2][3] = {};
+    for (size_t q = 0; q < p->seg_f.size(); ++q) a.tables |= ++count[p->seg_f[q]][p->seg_a[q]] > 2;
+    if (!a.tables) TFD_CHECK(slab_bounds(p, a.slab));
+    constexpr int N = Pack<T>::N;
+    const int groups = (a.g.n[0] + N - 1) / N;
+    auto magic = [](int d) { return d <= 1 ? 0xffffffffu : (unsigned)(((1ull << 32) + d - 1) / d); };
+    for (int f = 0; f < 2; ++f) {
+        // The longest run of groups that meet no x slab is the plain one.
+        std::vector<char> slab(groups, 0);
+        for (size_t q = 0; q < p->seg_f.size(); ++q)
+            if (p->seg_f[q] == f && p->seg_a[q] == 0)
+                for (int x = p->seg_lo[q]; x < p->seg_hi[q]; ++x) slab[x / N] = 1;
+        int from = 0, len = 0;
+        for (int x = 0; x < groups; ++x) {
+            int e = x;
+            while (e < groups && !slab[e]) ++e;
+            if (e - x > len) { from = x; len = e - x; }
+            x = std::max(x, e);
+        }
+        auto &sp = a.split[f];
+        sp.plain = len;
+        sp.x_lo = from;
+        sp.groups = groups;
+        sp.slab = groups - len;
+        sp.magic_plain = magic(sp.plain);
+        sp.magic_slab = magic(sp.slab);
+        sp.plain_total = (unsigned)sp.plain * a.g.n[1];
+        sp.total = (unsigned)groups * a.g.n[1];
+    }
+    p->pass_metric = false;
+    for (int f = 0; f < 2; ++f)
+        for (int ax = 0; ax < 3; ++ax) {
+            p->pass_metric = p->pass_metric || a.g.metric[f][ax] != nullptr;
+            p->pass_wide = p->pass_wide || a.g.count >= (1LL << 31) || p->L.psi_len[f][ax] >= (1LL << 31);
+        }
+    return setup_pass_steps<T>(p);
+}
+
+// One pass (E, or H from the stored E_new) of the two-pass step. Arrays of 2^31 elements and more take the variant with
+// 64-bit indices, which handles every other feature at run time.
+template <typename T, int ACTIVE>
+void launch_pass_active(tfd_plan *p, bool h, cudaStream_t s) {
+    const PassArgs<T> &a = p->pass<T>();
+    const dim3 grid((a.split[0].total + kPassThreads - 1) / kPassThreads, (unsigned)std::min(a.g.n[2], 65535));
+    const bool ade = a.g.n_ade > 0;
+    if (p->pass_wide) {
+        if (h) k_pass_h<T, ACTIVE, true, long long><<<grid, kPassThreads, 0, s>>>(a);
+        else k_pass_e<T, ACTIVE, true, true, long long><<<grid, kPassThreads, 0, s>>>(a);
+    } else if (h) {
+        if (p->pass_metric) k_pass_h<T, ACTIVE, true, int><<<grid, kPassThreads, 0, s>>>(a);
+        else k_pass_h<T, ACTIVE, false, int><<<grid, kPassThreads, 0, s>>>(a);
+    } else if (ade) {
+        if (p->pass_metric) k_pass_e<T, ACTIVE, true, true, int><<<grid, kPassThreads, 0, s>>>(a);
+        else k_pass_e<T, ACTIVE, false, true, int><<<grid, kPassThreads, 0, s>>>(a);
+    } else {
+        if (p->pass_metric) k_pass_e<T, ACTIVE, true, false, int><<<grid, kPassThreads, 0, s>>>(a);
+        else k_pass_e<T, ACTIVE, false, false, int><<<grid, kPassThreads, 0, s>>>(a);
+    }
+}
+
+template <typename T>
+void launch_pass(tfd_plan *p, bool h, cudaStream_t s) {
+    switch (p->grid<T>().active) {
+        case kMaskTM: launch_pass_active<T, kMaskTM>(p, h, s); break;
+        case kMaskTE: launch_pass_active<T, kMaskTE>(p, h, s); break;
+        default: launch_pass_active<T, kMaskAll>(p, h, s); break;
+    }
 }
 
 // The on-chip cluster path for small 2D TMz plans without DFT planes (TFD_CLUSTER2D=0 in the environment
@@ -1611,11 +1792,15 @@ int launch_persist2d(tfd_plan *p, int nsteps, cudaStream_t s) {
     return TFD_OK;
 }
 
-// One split step (plans with TFSF boxes or dispersive materials): the split gather E kernel, the boxes' E half
-// step and E corrections, the split gather H kernel, the H half step and H corrections (the observation launch
-// follows in step_t).
+// One two-pass step: the E pass, the TFSF boxes' E half step and E corrections, the H pass, the H half step and H
+// corrections (the observation launch follows in step_t).
 template <typename T>
-int launch_split_step(tfd_plan *p, cudaStream_t s) {
+int launch_two_pass(tfd_plan *p, cudaStream_t s) {
+    launch_pass<T>(p, false, s);
+    if (p->desc.n_tfsf == 0) {
+        launch_pass<T>(p, true, s);
+        return TFD_OK;
+    }
     const Grid<T> &g = p->grid<T>();
     TfsfArgs<T> a = p->tfsf<T>();
     for (int par = 0; par < 2; ++par)
@@ -1627,19 +1812,9 @@ int launch_split_step(tfd_plan *p, cudaStream_t s) {
     int longest = 1;
     for (int k = 0; k < a.boxes; ++k) longest = std::max(longest, a.box[k].count + std::max(a.box[k].n[0], a.box[k].n[1]));
     const dim3 tgrid((unsigned)((longest + kTfsfThreads - 1) / kTfsfThreads), (unsigned)a.boxes);
-    dim3 block(128), grid((unsigned)((long long)g.n[1] * g.n[2]), (unsigned)((g.n[0] + 127) / 128));
-    switch (g.active) {
-        case kMaskTM: k_step_gather_e<T, kMaskTM><<<grid, block, 0, s>>>(g); break;
-        case kMaskTE: k_step_gather_e<T, kMaskTE><<<grid, block, 0, s>>>(g); break;
-        default: k_step_gather_e<T, kMaskAll><<<grid, block, 0, s>>>(g); break;
-    }
-    if (a.boxes > 0) k_tfsf<T><<<tgrid, kTfsfThreads, 0, s>>>(a, 0);
-    switch (g.active) {
-        case kMaskTM: k_step_gather_h<T, kMaskTM><<<grid, block, 0, s>>>(g); break;
-        case kMaskTE: k_step_gather_h<T, kMaskTE><<<grid, block, 0, s>>>(g); break;
-        default: k_step_gather_h<T, kMaskAll><<<grid, block, 0, s>>>(g); break;
-    }
-    if (a.boxes > 0) k_tfsf<T><<<tgrid, kTfsfThreads, 0, s>>>(a, 1);
+    k_tfsf<T><<<tgrid, kTfsfThreads, 0, s>>>(a, 0);
+    launch_pass<T>(p, true, s);
+    k_tfsf<T><<<tgrid, kTfsfThreads, 0, s>>>(a, 1);
     return TFD_OK;
 }
 
@@ -1653,18 +1828,19 @@ int step_t(tfd_plan *p, int nsteps, cudaStream_t s) {
         if (nsteps > 0) TFD_CHECK(launch_persist2d<T>(p, nsteps, s));
         return TFD_OK;
     }
+    if (p->two_pass && p->pass_ctas > 0) {
+        if (nsteps > 0) TFD_CHECK(launch_pass_steps<T>(p, nsteps, s));
+        return TFD_OK;
+    }
     const MonitorArgs<T> m = monitor_args<T>(p);
     dim3 mgrid((unsigned)std::max(1, (p->max_samples + kMonitorThreads - 1) / kMonitorThreads), (unsigned)std::max(1, p->desc.n_planes));
     for (int k = 0; k < nsteps; ++k) {
-        if (p->split) {
-            TFD_CHECK(launch_split_step<T>(p, s));
+        if (p->two_pass) {
+            TFD_CHECK(launch_two_pass<T>(p, s));
         } else if (p->kernel == TFD_KERNEL_MARCH) {
             launch_march_any<T>(p, s);
-        } else if (p->kernel == TFD_KERNEL_TILE2D) {
-            launch_tile2d<T>(p, s);
         } else {
-            int rc = launch_step_gather<T>(p, s);
-            if (rc) return rc;
+            launch_tile2d<T>(p, s);
         }
         k_monitor<T><<<mgrid, kMonitorThreads, 0, s>>>(m);
     }
@@ -1845,12 +2021,14 @@ int tfd_plan_create(const tfd_desc *desc, void *arena, size_t arena_bytes, void 
             rc = fail(TFD_ERR_UNSUPPORTED, "the 2D tile kernel needs a 2D TMz grid without periodic x/y faces");
         p->split = desc->n_tfsf > 0 || desc->n_ade > 0;
         if (p->split && (desc->kernel == TFD_KERNEL_MARCH || desc->kernel == TFD_KERNEL_TILE2D))
-            rc = fail(TFD_ERR_UNSUPPORTED, "plans with TFSF boxes or dispersive materials run the split gather kernels");
+            rc = fail(TFD_ERR_UNSUPPORTED, "plans with TFSF boxes or dispersive materials run the two-pass step");
         if (desc->kernel == TFD_KERNEL_GATHER || p->split) p->kernel = TFD_KERNEL_GATHER;
         else if (march_ok) p->kernel = TFD_KERNEL_MARCH;
         else if (tile_ok) p->kernel = TFD_KERNEL_TILE2D;
         else p->kernel = TFD_KERNEL_GATHER;
         if (!rc && p->kernel == TFD_KERNEL_MARCH) rc = TFD_DISPATCH(p, setup_march, p);
+        p->two_pass = p->kernel == TFD_KERNEL_GATHER || (p->kernel == TFD_KERNEL_MARCH && two_pass_3d(p));
+        if (!rc && p->two_pass) rc = TFD_DISPATCH(p, setup_pass, p);
         if (!rc && tile_ok && !p->split) rc = TFD_DISPATCH(p, setup_tile2d, p, s);
     }
     if (!rc) rc = TFD_DISPATCH(p, zero_state, p, s);
@@ -1987,16 +2165,18 @@ int tfd_kernel_in_use(const tfd_plan *p, int32_t *kernel) {
 int tfd_step_launches(const tfd_plan *p, int32_t nsteps, int64_t *launches) {
     if (!p || !launches) return fail(TFD_ERR_INVALID, "null argument");
     if (nsteps < 0) return fail(TFD_ERR_INVALID, "nsteps must be non-negative");
-    long long per_step = 2;                                   // gather: step + observation
-    if (p->split) {
-        per_step = p->desc.n_tfsf > 0 ? 5 : 3;                // split E, (TFSF E), split H, (TFSF H), observation
-    } else if (p->kernel == TFD_KERNEL_TILE2D) {
+    if (p->two_pass && p->pass_ctas > 0) {
+        *launches = nsteps > 0 ? 1 : 0;
+        return TFD_OK;
+    }
+    long long per_step = p->desc.n_tfsf > 0 ? 5 : 3;         // two passes: E, (TFSF E), H, (TFSF H), observation
+    if (!p->two_pass && p->kernel == TFD_KERNEL_TILE2D) {
         if ((p->persist_ctas > 0 || p->cluster2d.ranks > 0) && !p->in_batch) {
             *launches = nsteps > 0 ? 1 : 0;
             return TFD_OK;
         }
         per_step = (p->tile2d_interior > 0) + (p->L.tiles2d > p->tile2d_interior) + 1;
-    } else if (p->kernel == TFD_KERNEL_MARCH) {
+    } else if (!p->two_pass && p->kernel == TFD_KERNEL_MARCH) {
         per_step = (long long)p->march_launches.size() + 1;
     }
     *launches = per_step * nsteps;

@@ -15,7 +15,7 @@
 // chunks are independent. E and H are double-buffered in HBM (ping-pong over steps),
 // so a halo value is recomputed from the same old inputs with the same arithmetic as
 // by its owner: bitwise identical, no inter-CTA synchronisation. The arithmetic is the
-// reference operation order (see step_gather.cuh). Global traffic per cell: one read
+// reference operation order (see step_pass.cuh). Global traffic per cell: one read
 // and one write of each field component, one read of the permittivity, and the CPML
 // memories of slab cells only; halos are re-read from L2.
 //

@@ -10,8 +10,8 @@
 // reference order (torchfdtd/tfsf.py:125-176, torchfdtd/cuda_tfsf.py:19-49): psi = psi*b + c*diff;
 // line -= factor*(diff + psi); field += weight*incident.
 //
-// The grid's E and H updates run as the split gather kernels (k_step_gather_e / k_step_gather_h) so that
-// the E corrections land before the H update reads E.
+// The grid's E and H updates run as two passes (step_pass.cuh), so that the E corrections land before the H pass
+// reads E.
 #pragma once
 #include "internal.cuh"
 

@@ -82,12 +82,13 @@ def _interleaved(runners, repeats, steps, stream):
 
 
 def grid_candidates(plan):
-    """Marching-kernel launch variants worth measuring for a plan."""
+    """Launch variants worth measuring for a 3D plan: 0 (the default, which steps in two passes on all but the largest
+    uniform FP32 grids) and the marching kernel's own."""
     nz = plan.shape[2]
     if plan.dtype == np.float64:
-        base = [22, 122]
+        base = [0, 22, 122]
     else:
-        base = [14, 23, 32, 22, 114, 314]
+        base = [0, 14, 23, 32, 22, 114, 314]
     lz = [v for v in (4, 8, 16) if v < nz]            # planes per chunk around the default (about 12)
     return base + [z * 1000 + 14 for z in lz] if plan.dtype != np.float64 else base + [z * 1000 + 22 for z in lz]
 
