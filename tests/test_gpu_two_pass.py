@@ -1,12 +1,13 @@
-"""The two-pass step kernels against the NumPy oracle: every way they are launched (three launches per step, one cluster,
+"""The two-pass step kernels and the reverse step's two passes against the NumPy oracle: every way they are launched (three launches per step, one cluster,
 one cooperative launch), at row lengths around the 16-byte groups, and with more than two CPML slabs on an axis (the
-row-table path). Bar: fields, CPML memories and traces bitwise, like the other step kernels (same operations, same
-order, no contraction)."""
+row-table path). Bars: fields, CPML memories and traces bitwise, like the other step kernels (same operations, same
+order, no contraction); gradients within the relative L2 of tests/test_gpu_adjoint.py."""
 from dataclasses import replace
 
 import numpy as np
 import pytest
 
+from oracle.adjoint_oracle import AdjointOracle
 from oracle.yee_oracle import YeeOracle
 from torchfdtd_b200 import Project, Region
 from torchfdtd_b200.models import BoundaryFace, Monitor, Source
@@ -91,3 +92,29 @@ def test_default_3d_step_equals_the_marching_kernel(shape, steps):
         grid.close()
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize('shape,precision,faces,component', [
+    ((13, 14, 15), 'float32', None, 'Ey'), ((14, 13, 16), 'float64', {'z_max': BoundaryFace(kind='pec')}, 'Hz'),
+    ((17, 15, 13), 'float64', {**PERIODIC_Y, 'x_max': BoundaryFace(kind='pec')}, 'Ez'),
+    ((15, 16, 13), 'float64', {'x_min': BoundaryFace(kind='periodic'), 'x_max': BoundaryFace(kind='periodic')}, 'Ez'),
+    ((65, 33, 1), 'float32', PERIODIC_Y, 'Hz'), ((34, 40, 1), 'float64', None, 'Ez')])
+def test_reverse_step_matches_the_oracle(shape, precision, faces, component):
+    import torch
+    from torchfdtd_b200.adjoint import DifferentiableSimulation
+    project = scene(shape, precision, faces, component, steps=24)
+    plan = plan_grid(project)
+    rng = np.random.default_rng(8)
+    eps = rng.uniform(1, 3, size=plan.shape)
+    w = rng.normal(size=(plan.steps, 1))
+    dtype = torch.float32 if precision == 'float32' else torch.float64
+    model = DifferentiableSimulation(project)
+    epsilon = torch.tensor(eps, dtype=dtype, device='cuda', requires_grad=True)
+    result = model(epsilon)
+    (result.signals * torch.tensor(w, dtype=dtype, device='cuda')).sum().backward()
+    oracle = AdjointOracle(plan, eps.astype(plan.dtype))
+    np.testing.assert_array_equal(result.signals.detach().cpu().numpy(), oracle.forward())
+    want = oracle.backward(w.astype(plan.dtype))
+    got = epsilon.grad.cpu().numpy()
+    assert np.linalg.norm(got - want) <= (1e-5 if precision == 'float32' else 1e-11) * np.linalg.norm(want) and np.linalg.norm(want) > 0
+    model.close()

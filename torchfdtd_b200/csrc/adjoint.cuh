@@ -16,19 +16,20 @@
 //
 // curl_f^T is a backward difference of the per-H-cell values D(k) (k = 0..n-2, plus the periodic wrap or
 // PEC edge at n-1) and curl_b^T a forward difference of per-E-cell values D(k) (k = 1..n-1, plus the
-// periodic edge at 0), so the adjoint step has the forward step's stencil shape. It runs as two
-// launches, one thread per cell: k_adjoint_e writes e_bar_new (and accumulates the sensitivity),
-// k_adjoint_h reads e_bar_new of its own cell and its +x, +y, +z neighbours back and writes h_bar_new.
-// (A single launch that recomputes the neighbours' e_bar_new, as the forward gather kernel recomputes E,
-// ran about 4x slower: each h_bar term needs a neighbour's e_bar, which needs CPML-transposed D values
-// at two cells.) Adjoint fields and both families' adjoint CPML memories are double-buffered by
-// reverse-step parity; each memory is written once, by the thread that owns its cell. The forward state comes from a restart snapshot (tfd_state_save)
-// of s_n, so no forward buffer is disturbed.
+// periodic edge at 0), so the adjoint step has the forward step's stencil shape and runs like it as two passes, one
+// thread per 16-byte group of cells: k_adjoint_e writes e_bar_new (and accumulates the sensitivity), k_adjoint_h reads
+// e_bar_new of its own cells and their +x, +y, +z neighbours back and writes h_bar_new. Adjoint fields and both
+// families' adjoint CPML memories are double-buffered by reverse-step parity; each memory is written once, by the thread
+// that owns its cell. The forward state comes from a snapshot of s_n, so no forward buffer is disturbed.
+//
+// What bounds them on large grids is DRAM: in FP32 60 bytes per cell in the E pass (h_bar, the snapshot's H, e_bar and S
+// read, e_bar and S written) and 40 in the H pass.
 //
 // The material sensitivity is accumulated as S_c = sum_n e_bar_c * curl_b(H)_c per component; the host
 // forms dJ/d eps = -cn S / eps^2 (summed over components for a per-cell permittivity).
 #pragma once
 #include "internal.cuh"
+#include "step_pass.cuh"
 
 namespace tfd {
 
@@ -50,6 +51,7 @@ struct AdjArgs {
     T *pEb[2][3][2], *pHb[2][3][2];   // adjoint CPML memories [parity][axis][term j]
     T *S[3];                     // material sensitivity per E component
     int slab[2][3][4];           // per family and axis: lo0, hi0, lo1, hi1 of the two CPML slabs
+    PassSplit split;             // groups of a row away from the x slabs, and the others
 };
 
 // Slab row of coordinate c from the (lo, hi) bounds of a (family, axis), or -1: rows of the low slab first.
@@ -58,401 +60,355 @@ __device__ __forceinline__ int adj_slab_row(const int *b, int c) {
     return (c >= b[0] && c < b[1]) ? c - b[0] : (c >= b[2] && c < b[3]) ? (b[1] - b[0]) + (c - b[2]) : -1;
 }
 
-template <typename T>
-__device__ __forceinline__ int coord_of(int a, int x, int y, int z) { return a == 0 ? x : (a == 1 ? y : z); }
-
-// D of an H-family term (output H component `out`, axis a) at H cell k: the transposed forward-difference
-// value sign * (-cn h_bar_out[k]) through the CPML memory transpose. Writes the memory when own.
-template <typename T>
-__device__ __forceinline__ T d_h(const AdjArgs<T> &A, int q, const RevTerm t, int x, int y, int z, long long k, bool own) {
+// CPML transpose of the D values v[] of a group's cells in one y or z slab row r: m = psi_bar + v; psi_bar <- b m (when
+// own); v <- v / kappa + c m.
+template <typename T, int F, int a>
+__device__ __forceinline__ void adj_slab_row_apply(const AdjArgs<T> &A, int r, int x, int y, int z, const T *old, T *out, bool own,
+                                                   T (&v)[Pack<T>::N]) {
+    constexpr int N = Pack<T>::N;
     const Grid<T> &g = A.g;
-    const int a = t.axis;
-    const int c = coord_of<T>(a, x, y, z);
-    const T dst = -g.cn * A.hb[q][t.out][k];
-    T v = t.sign > 0 ? dst : -dst;
-    const T *mt = g.metric[1][a];
-    if (c < g.n[a] - 1) {
-        if (A.pHb[q][a][t.j] != nullptr) {
-            const int r = adj_slab_row(A.slab[1][a], c);
-            if (r >= 0) {
-                const long long p = g.psi_index(a, x, y, z, r, g.rows[1][a]);
-                const T m = A.pHb[q][a][t.j][p] + v;
-                if (own) A.pHb[q ^ 1][a][t.j][p] = g.cb[1][a][c] * m;
-                v = v * g.ck[1][a][c] + g.cc[1][a][c] * m;
-            }
-        }
-        return mt != nullptr ? v * mt[c] : v;       // the forward scales before its CPML terms
-    }
-    if (g.periodic[a]) return mt != nullptr ? v * mt[c] : v;
-    if (g.pec_on[a]) return -g.pec_neg[a] * v;       // sign * pec * dst
-    return T(0);
-}
-
-// e_bar_new of component C at cell (x, y, z), index i.
-template <typename T, int C>
-__device__ __forceinline__ T ebar_value(const AdjArgs<T> &A, int q, int x, int y, int z, long long i, bool own) {
-    const Grid<T> &g = A.g;
-    T contrib = T(0);
+    const int c = a == 1 ? y : z;
+    const long long p = g.psi_index(a, x, y, z, r, g.rows[F][a]);
+    const T b = g.cb[F][a][c], cc = g.cc[F][a][c], ck = g.ck[F][a][c];
+    const Pack<T> m0 = pack_load(old + p);
+    Pack<T> w;
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const RevTerm t = rev_of(C, k);
-        const int a = t.axis;
-        if (g.n[a] == 1) continue;
-        const int out_bit = 1 << (3 + t.out);
-        if (!(g.active & out_bit)) continue;
-        const int c = coord_of<T>(a, x, y, z);
-        const int n = g.n[a];
-        const long long s = g.stride(a);
-        if (c >= 1) {                                   // src[c] += D(c-1)
-            const int xm = a == 0 ? x - 1 : x, ym = a == 1 ? y - 1 : y, zm = a == 2 ? z - 1 : z;
-            contrib = contrib + d_h(A, q, t, xm, ym, zm, i - s, false);
-        }
-        if (c <= n - 2) contrib = contrib - d_h(A, q, t, x, y, z, i, own);   // src[c] -= D(c)
-        if (g.periodic[a]) {                            // wrap edge D(n-1): src[0] += D, src[n-1] -= D
-            if (c == 0) {
-                const int xw = a == 0 ? n - 1 : x, yw = a == 1 ? n - 1 : y, zw = a == 2 ? n - 1 : z;
-                contrib = contrib + d_h(A, q, t, xw, yw, zw, i + (long long)(n - 1) * s, false);
-            }
-            if (c == n - 1) contrib = contrib - d_h(A, q, t, x, y, z, i, false);
-        } else if (g.pec_on[a] && c == n - 1) {
-            contrib = contrib - d_h(A, q, t, x, y, z, i, false);
-        }
+    for (int k = 0; k < N; ++k) {
+        const T m = m0.v[k] + v[k];
+        w.v[k] = b * m;
+        v[k] = v[k] * ck + cc * m;
     }
-    return A.eb[q][C][i] + contrib;
+    if (own) pack_store(out + p, w);
 }
 
-// D of an E-family term (output E component `out`, axis a) at E cell k: sign * (cn / eps) e_bar_new_out[k]
-// through the CPML memory transpose. Writes the memory when own.
-template <typename T>
-__device__ __forceinline__ T d_e(const AdjArgs<T> &A, int q, const RevTerm t, int x, int y, int z, long long k, T ebar_out,
-                                 bool own) {
+// The same for one cell of an x slab.
+template <typename T, int F>
+__device__ __forceinline__ T adj_slab_x_apply(const AdjArgs<T> &A, int x, int y, int z, const T *old, T *out, bool own, T v) {
     const Grid<T> &g = A.g;
-    const int a = t.axis;
-    const int c = coord_of<T>(a, x, y, z);
-    const T dst = (g.cn * g.inv_eps[t.out][k]) * ebar_out;
-    T v = t.sign > 0 ? dst : -dst;
-    const T *mt = g.metric[0][a];
-    if (c >= 1) {
-        if (A.pEb[q][a][t.j] != nullptr) {
-            const int r = adj_slab_row(A.slab[0][a], c);
-            if (r >= 0) {
-                const long long p = g.psi_index(a, x, y, z, r, g.rows[0][a]);
-                const T m = A.pEb[q][a][t.j][p] + v;
-                if (own) A.pEb[q ^ 1][a][t.j][p] = g.cb[0][a][c] * m;
-                v = v * g.ck[0][a][c] + g.cc[0][a][c] * m;
-            }
-        }
-        return mt != nullptr ? v * mt[c] : v;
-    }
-    return g.periodic[a] ? (mt != nullptr ? v * mt[0] : v) : T(0);
+    if (old == nullptr || x < 0 || x >= g.n[0]) return v;
+    const int r = adj_slab_row(A.slab[F][0], x);
+    if (r < 0) return v;
+    const long long p = g.psi_index(0, x, y, z, r, g.rows[F][0]);
+    const T m = old[p] + v;
+    if (own) out[p] = g.cb[F][0][x] * m;
+    return v * g.ck[F][0][x] + g.cc[F][0][x] * m;
 }
 
-template <typename T, int C>
-__device__ __forceinline__ T ebar_at(const AdjArgs<T> &A, int q, int x, int y, int z, long long i) {
-    return ebar_value<T, C>(A, q, x, y, z, i, false);
-}
-
-// e_bar_new of component `out` at a neighbour (runtime component).
-template <typename T>
-__device__ __forceinline__ T ebar_any(const AdjArgs<T> &A, int q, int out, int x, int y, int z, long long i) {
-    return out == 0 ? ebar_at<T, 0>(A, q, x, y, z, i) : out == 1 ? ebar_at<T, 1>(A, q, x, y, z, i) : ebar_at<T, 2>(A, q, x, y, z, i);
-}
-
-// h_bar_new of H component C at its own cell; e_own[] holds e_bar_new of the own cell. STORED: the
-// neighbours' e_bar_new are read from the new buffer (written by k_adjoint_e) instead of recomputed.
-template <typename T, int C, bool STORED = false>
-__device__ __forceinline__ T hbar_value(const AdjArgs<T> &A, int q, int x, int y, int z, long long i, const T *e_own) {
+// e_bar_new and the sensitivity of a group. XS: the group or a neighbour of its ends lies in an x slab.
+// The D values of H-family terms are sign * (-cn h_bar): through the CPML transpose below the last cell, one period away
+// or the PEC edge at it; e_bar[c] += D(c - 1), e_bar[c] -= D(c), in the order of the terms.
+template <typename T, int ACTIVE, bool XS>
+__device__ __forceinline__ void adj_pass_e(const AdjArgs<T> &A, const T *__restrict__ slot, int q, const PassCell<long long> &w) {
+    constexpr int N = Pack<T>::N;
     const Grid<T> &g = A.g;
-    T contrib = T(0);
+    const long long i = w.i;
+    const int x = w.x, y = w.y, z = w.z, nx = g.n[0], ny = g.n[1], nz = g.n[2];
+    const bool last = x + N >= nx;
+    const long long ix = x > 0 ? i - 1 : i + (g.periodic[0] ? nx - 1 : 0);
+    const long long iy = y > 0 ? i - g.pitch : i + (g.periodic[1] ? (long long)(ny - 1) * g.pitch : 0);
+    const long long iz = z > 0 ? i - g.plane : i + (g.periodic[2] ? (long long)(nz - 1) * g.plane : 0);
+    Pack<T> h[3], hy[3], hz[3], f[3], fy[3], fz[3], eb[3], S[3];
+    T hx[3], fx[3];
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const RevTerm t = rev_of(C, k);
-        const int a = t.axis;
-        if (g.n[a] == 1) continue;
-        if (!(g.active & (1 << t.out))) continue;
-        const int c = coord_of<T>(a, x, y, z);
-        const int n = g.n[a];
-        const long long s = g.stride(a);
-        if (c >= 1) contrib = contrib + d_e(A, q, t, x, y, z, i, e_own[t.out], true);          // src[c] += D(c)
-        if (c + 1 <= n - 1) {                                                                   // src[c] -= D(c+1)
-            const int xp = a == 0 ? x + 1 : x, yp = a == 1 ? y + 1 : y, zp = a == 2 ? z + 1 : z;
-            const T eb = STORED ? A.eb[q ^ 1][t.out][i + s] : ebar_any(A, q, t.out, xp, yp, zp, i + s);
-            contrib = contrib - d_e(A, q, t, xp, yp, zp, i + s, eb, false);
+    for (int c = 0; c < 3; ++c) {
+        h[c] = hy[c] = hz[c] = f[c] = fy[c] = fz[c] = eb[c] = S[c] = Pack<T>{};
+        hx[c] = fx[c] = T(0);
+        if ((ACTIVE >> (3 + c)) & 1) {
+            const T *hb = A.hb[q][c], *sf = slot + A.sH[c];
+            h[c] = pack_load(hb + i);
+            f[c] = pack_load(sf + i);
+            if (c != 0) { hx[c] = hb[ix]; fx[c] = sf[ix]; }
+            if (c != 1 && ny > 1) { hy[c] = pack_load(hb + iy); fy[c] = pack_load(sf + iy); }
+            if (c != 2 && nz > 1) { hz[c] = pack_load(hb + iz); fz[c] = pack_load(sf + iz); }
         }
-        if (g.periodic[a]) {                             // edge D(0): src[0] += D, src[n-1] -= D
-            if (c == 0) contrib = contrib + d_e(A, q, t, x, y, z, i, e_own[t.out], false);
-            if (c == n - 1) {
-                const int x0 = a == 0 ? 0 : x, y0 = a == 1 ? 0 : y, z0 = a == 2 ? 0 : z;
-                const long long i0 = i - (long long)(n - 1) * s;
-                const T eb = STORED ? A.eb[q ^ 1][t.out][i0] : ebar_any(A, q, t.out, x0, y0, z0, i0);
-                contrib = contrib - d_e(A, q, t, x0, y0, z0, i0, eb, false);
-            }
+        if ((ACTIVE >> c) & 1) {
+            eb[c] = pack_load(A.eb[q][c] + i);
+            S[c] = pack_load(A.S[c] + i);
         }
     }
-    return A.hb[q][C][i] + contrib;
-}
-
-// Forward E curl of component C from the snapshot (same arithmetic as the forward E update).
-template <typename T, int C>
-__device__ __forceinline__ T forward_curl(const AdjArgs<T> &A, const T *slot, int x, int y, int z, long long i) {
-    const Grid<T> &g = A.g;
-    T acc = T(0);
+    const bool metric = g.metric[0][0] != nullptr || g.metric[0][1] != nullptr || g.metric[0][2] != nullptr;
+    auto mt = [&](int fam, int a, int c) -> T { return g.metric[fam][a] != nullptr ? g.metric[fam][a][c] : T(1); };
+    Pack<T> e[3];
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const Term t = term_of(C, k);
-        const int a = t.axis;
-        if (g.n[a] == 1) continue;
-        const int c = coord_of<T>(a, x, y, z);
-        const T *h = slot + A.sH[t.in];
-        const T *mt = g.metric[0][a];
-        T d = T(0);
-        if (c > 0) {
-            d = h[i] - h[i - g.stride(a)];
-            if (mt != nullptr) d = d * mt[c];
+    for (int C = 0; C < 3; ++C) {
+        if (!((ACTIVE >> C) & 1)) continue;
+        T contrib[N], acc[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) contrib[k] = acc[k] = T(0);
+#pragma unroll
+        for (int t2 = 0; t2 < 2; ++t2) {
+            const RevTerm t = rev_of(C, t2);
+            const int a = t.axis, o = t.out;
+            if (g.n[a] == 1 || !((ACTIVE >> (3 + o)) & 1)) continue;
+            // D at the cells below (lo) and at the cells themselves (up).
+            T lo[N], up[N];
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                const T below = a == 0 ? (k == 0 ? hx[o] : h[o].v[k == 0 ? 0 : k - 1]) : a == 1 ? hy[o].v[k] : hz[o].v[k];
+                const T dl = -g.cn * below, du = -g.cn * h[o].v[k];
+                lo[k] = t.sign > 0 ? dl : -dl;
+                up[k] = t.sign > 0 ? du : -du;
+            }
+            const T *old = A.pHb[q][a][t.j];
+            T *out = A.pHb[q ^ 1][a][t.j];
+            if (a == 0) {
+#pragma unroll
+                for (int k = 0; k < N; ++k) {
+                    const int c = x + k;
+                    if (XS) {
+                        if (c >= 1) lo[k] = adj_slab_x_apply<T, 1>(A, c - 1, y, z, old, out, false, lo[k]);
+                        if (c < nx - 1) up[k] = adj_slab_x_apply<T, 1>(A, c, y, z, old, out, true, up[k]);
+                    }
+                    if (metric && c < nx) {
+                        lo[k] = lo[k] * mt(1, 0, c >= 1 ? c - 1 : nx - 1);
+                        if (c < nx - 1 || g.periodic[0]) up[k] = up[k] * mt(1, 0, c);
+                    }
+                    if (k == 0 && x == 0) {
+                        // No cell below: nothing, or the wrap edge, added after the own cell's value.
+                        contrib[0] = contrib[0] - up[0];
+                        if (g.periodic[0]) contrib[0] = contrib[0] + lo[0];
+                        continue;
+                    }
+                    contrib[k] = contrib[k] + lo[k];
+                    if (!last || c < nx - 1) contrib[k] = contrib[k] - up[k];
+                    else if (c == nx - 1) {
+                        if (g.periodic[0]) contrib[k] = contrib[k] - up[k];
+                        else if (g.pec_on[0]) contrib[k] = contrib[k] - (-g.pec_neg[0] * up[k]);
+                    }
+                }
+            } else {
+                const int c = a == 1 ? y : z, n = g.n[a];
+                if (c >= 1 && old != nullptr) {
+                    const int r = adj_slab_row(A.slab[1][a], c - 1);
+                    if (r >= 0) {
+                        if (a == 1) adj_slab_row_apply<T, 1, 1>(A, r, x, y - 1, z, old, out, false, lo);
+                        else adj_slab_row_apply<T, 1, 2>(A, r, x, y, z - 1, old, out, false, lo);
+                    }
+                }
+                if (c < n - 1 && old != nullptr) {
+                    const int r = adj_slab_row(A.slab[1][a], c);
+                    if (r >= 0) {
+                        if (a == 1) adj_slab_row_apply<T, 1, 1>(A, r, x, y, z, old, out, true, up);
+                        else adj_slab_row_apply<T, 1, 2>(A, r, x, y, z, old, out, true, up);
+                    }
+                }
+                const T ml = metric ? mt(1, a, c >= 1 ? c - 1 : n - 1) : T(1), mu = metric ? mt(1, a, c) : T(1);
+                const bool pec = c == n - 1 && !g.periodic[a] && g.pec_on[a], none = c == n - 1 && !g.periodic[a] && !g.pec_on[a];
+#pragma unroll
+                for (int k = 0; k < N; ++k) {
+                    if (metric) {
+                        lo[k] = lo[k] * ml;
+                        if (!pec) up[k] = up[k] * mu;
+                    }
+                    if (pec) up[k] = -g.pec_neg[a] * up[k];
+                    if (c >= 1) contrib[k] = contrib[k] + lo[k];
+                    if (!none) contrib[k] = contrib[k] - up[k];
+                    if (c == 0 && g.periodic[a]) contrib[k] = contrib[k] + lo[k];
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < N; ++k) e[C].v[k] = eb[C].v[k] + contrib[k];
+        // The forward E curl from the snapshot (the arithmetic of the forward E update).
+#pragma unroll
+        for (int t2 = 0; t2 < 2; ++t2) {
+            const Term t = term_of(C, t2);
+            const int a = t.axis, in = t.in;
+            if (g.n[a] == 1) continue;
+            T d[N];
+            const int c0 = a == 0 ? x : a == 1 ? y : z;
+            const bool live = c0 > 0 || g.periodic[a];
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                const T below = a == 0 ? (k == 0 ? fx[in] : f[in].v[k == 0 ? 0 : k - 1]) : a == 1 ? fy[in].v[k] : fz[in].v[k];
+                d[k] = f[in].v[k] - below;
+                if ((a != 0 || k == 0) && !live) d[k] = T(0);
+                if (metric) d[k] = d[k] * mt(0, a, a == 0 ? min(x + k, nx - 1) : c0);
+            }
             if (A.sPsiE[a][t.j] >= 0) {
-                const int r = adj_slab_row(A.slab[0][a], c);
-                if (r >= 0) {
-                    const long long p = g.psi_index(a, x, y, z, r, g.rows[0][a]);
-                    const T mem = slot[A.sPsiE[a][t.j] + p] * g.cb[0][a][c] + g.cc[0][a][c] * d;
-                    d = d * g.ck[0][a][c] + mem;
+                const T *psi = slot + A.sPsiE[a][t.j];
+                if (a == 0) {
+                    if (XS)
+#pragma unroll
+                        for (int k = 0; k < N; ++k) {
+                            const int c = x + k, r = c < nx ? adj_slab_row(A.slab[0][0], c) : -1;
+                            if (c > 0 && r >= 0) {
+                                const T m = psi[g.psi_index(0, c, y, z, r, g.rows[0][0])] * g.cb[0][0][c] + g.cc[0][0][c] * d[k];
+                                d[k] = d[k] * g.ck[0][0][c] + m;
+                            }
+                        }
+                } else {
+                    const int r = c0 > 0 ? adj_slab_row(A.slab[0][a], c0) : -1;
+                    if (r >= 0) {
+                        const Pack<T> m0 = pack_load(psi + g.psi_index(a, x, y, z, r, g.rows[0][a]));
+                        const T b = g.cb[0][a][c0], cc = g.cc[0][a][c0], ck = g.ck[0][a][c0];
+#pragma unroll
+                        for (int k = 0; k < N; ++k) {
+                            const T m = m0.v[k] * b + cc * d[k];
+                            d[k] = d[k] * ck + m;
+                        }
+                    }
                 }
             }
-        } else if (g.periodic[a]) {
-            d = h[i] - h[i + (long long)(g.n[a] - 1) * g.stride(a)];
-            if (mt != nullptr) d = d * mt[0];
+#pragma unroll
+            for (int k = 0; k < N; ++k) acc[k] = acc[k] + (t.sign > 0 ? d[k] : -d[k]);
         }
-        acc = acc + (t.sign > 0 ? d : -d);
-    }
-    return acc;
-}
-
-// ACTIVE: bitmask of advanced components (bit c: E_c, bit 3+c: H_c). Blocks of kAdjX x kAdjY cells of one
-// z plane (blockIdx.x, blockIdx.y: x and y tile; blockIdx.z: plane), so the x and y neighbours a cell reads
-// are mostly in its block's L1 lines. The tile origins are shifted by (xs, ys) cells (tile (bx, by) starts at
-// (bx kAdjX - xs, by kAdjY - ys)) so that tiles start at x = 1 and y = 1; tiles clear of the grid faces take a
-// fast path unless `fast` is 0 (the general path alone, for comparisons). Reads parity q, writes q^1.
-constexpr int kAdjX = 32, kAdjY = 8;
-
-// Whether the CPML slab bounds b = {lo0, hi0, lo1, hi1} (half-open) meet the coordinates [lo, hi].
-__host__ __device__ __forceinline__ bool adj_meets(const int *b, int lo, int hi) {
-    return (lo < b[1] && b[0] <= hi) || (lo < b[3] && b[2] <= hi);
-}
-
-// Block classes for the fast paths. Every cell of the block lies in [1, n-2] on every axis (both neighbours
-// inside the grid: no face or periodic edge); otherwise the block takes the general path (class -1). Else the
-// class is a mask with bit a set when a CPML term may apply to a D value the block's cells evaluate on axis a:
-// the H family on [lo - 1, hi] (HFAM: the e_bar update differences D(c-1) and D(c)) and the E family on
-// [lo, hi + e_hi]. Terms on the axes of the mask go through the general D functions; the others are the plain
-// transposed differences, to which the general path's arithmetic reduces there, in the same order.
-template <typename T>
-__device__ __forceinline__ int adj_class(const AdjArgs<T> &A, int x0, int y0, int z, bool hfam, int e_hi) {
-    const Grid<T> &g = A.g;
-    const int lo[3] = {max(x0, 0), max(y0, 0), z};
-    const int hi[3] = {min(x0 + kAdjX, g.n[0]) - 1, min(y0 + kAdjY, g.n[1]) - 1, z};
-    int mask = 0;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        if (lo[a] < 1 || hi[a] > g.n[a] - 2) return -1;
-        if ((hfam && adj_meets(A.slab[1][a], lo[a] - 1, hi[a])) || adj_meets(A.slab[0][a], lo[a], hi[a] + e_hi)) mask |= 1 << a;
-    }
-    return mask;
-}
-
-// e_bar_new and the sensitivity of the three components of a cell of a fast-path block; GEN: the axes whose
-// terms go through the general D functions (the mask above). Every input of the plain terms is loaded before
-// the first store (the stores could alias the loads for the compiler, which would otherwise serialise the three
-// components' memory round trips).
-template <typename T, int GEN>
-__device__ __forceinline__ void adj_e_fast(const AdjArgs<T> &A, const T *__restrict__ slot, int q, int x, int y, int z, long long i) {
-    const Grid<T> &g = A.g;
-    const int co[3] = {x, y, z};
-    T hc[3], sc[3], hm[3][2], smv[3][2], eb[3], S0[3];
-#pragma unroll
-    for (int o = 0; o < 3; ++o) {
-        hc[o] = __ldg(A.hb[q][o] + i);
-        sc[o] = __ldg(slot + A.sH[o] + i);
-        eb[o] = __ldg(A.eb[q][o] + i);
-        S0[o] = A.S[o][i];
+        for (int k = 0; k < N; ++k) {
+            S[C].v[k] = S[C].v[k] + e[C].v[k] * acc[k];
+            if (x + k >= nx) e[C].v[k] = S[C].v[k] = T(0);
+        }
     }
 #pragma unroll
     for (int C = 0; C < 3; ++C)
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const RevTerm t = rev_of(C, k);
-            if (!((GEN >> t.axis) & 1)) hm[C][k] = __ldg(A.hb[q][t.out] + i - g.stride(t.axis));
-            const Term f = term_of(C, k);
-            smv[C][k] = __ldg(slot + A.sH[f.in] + i - g.stride(f.axis));
+        if ((ACTIVE >> C) & 1) {
+            pack_store(A.eb[q ^ 1][C] + i, e[C]);
+            pack_store(A.S[C] + i, S[C]);
         }
-    T e[3], s[3];
+}
+
+// h_bar_new of a group from the stored e_bar_new. The D values of E-family terms are sign * ((cn / eps) e_bar_new), zero
+// at cell 0 without a period; h_bar[c] += D(c), h_bar[c] -= D(c + 1).
+template <typename T, int ACTIVE, bool XS>
+__device__ __forceinline__ void adj_pass_h(const AdjArgs<T> &A, int q, const PassCell<long long> &w) {
+    constexpr int N = Pack<T>::N;
+    const Grid<T> &g = A.g;
+    const long long i = w.i;
+    const int x = w.x, y = w.y, z = w.z, nx = g.n[0], ny = g.n[1], nz = g.n[2];
+    const bool last = x + N >= nx;
+    const long long ix = last ? i - x : i + N;
+    const long long iy = y < ny - 1 ? i + g.pitch : i - (g.periodic[1] ? (long long)(ny - 1) * g.pitch : 0);
+    const long long iz = z < nz - 1 ? i + g.plane : i - (g.periodic[2] ? (long long)(nz - 1) * g.plane : 0);
+    // u = (cn / eps) e_bar_new at the cells and at the +x, +y, +z neighbours.
+    Pack<T> u[3], uy[3], uz[3], hb[3];
+    T ux[3];
+    auto scaled = [&](const Pack<T> &ie, const Pack<T> &eb) {
+        Pack<T> r;
+#pragma unroll
+        for (int k = 0; k < N; ++k) r.v[k] = (g.cn * ie.v[k]) * eb.v[k];
+        return r;
+    };
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        u[c] = uy[c] = uz[c] = hb[c] = Pack<T>{};
+        ux[c] = T(0);
+        if ((ACTIVE >> c) & 1) {
+            const T *eb = A.eb[q ^ 1][c], *ie = g.inv_eps[c];
+            u[c] = scaled(pack_load(ie + i), pack_load(eb + i));
+            if (c != 0) ux[c] = (g.cn * ie[ix]) * eb[ix];
+            if (c != 1 && ny > 1) uy[c] = scaled(pack_load(ie + iy), pack_load(eb + iy));
+            if (c != 2 && nz > 1) uz[c] = scaled(pack_load(ie + iz), pack_load(eb + iz));
+        }
+        if ((ACTIVE >> (3 + c)) & 1) hb[c] = pack_load(A.hb[q][c] + i);
+    }
+    const bool metric = g.metric[0][0] != nullptr || g.metric[0][1] != nullptr || g.metric[0][2] != nullptr;
+    auto mt = [&](int a, int c) -> T { return g.metric[0][a] != nullptr ? g.metric[0][a][c] : T(1); };
 #pragma unroll
     for (int C = 0; C < 3; ++C) {
-        T contrib = T(0);
+        if (!((ACTIVE >> (3 + C)) & 1)) continue;
+        T contrib[N];
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const RevTerm t = rev_of(C, k);
-            const int a = t.axis, c = co[a];
-            if ((GEN >> a) & 1) {
-                const int xm = a == 0 ? x - 1 : x, ym = a == 1 ? y - 1 : y, zm = a == 2 ? z - 1 : z;
-                contrib = contrib + d_h(A, q, t, xm, ym, zm, i - g.stride(a), false);   // src[c] += D(c-1)
-                contrib = contrib - d_h(A, q, t, x, y, z, i, true);                    // src[c] -= D(c)
-                continue;
+        for (int k = 0; k < N; ++k) contrib[k] = T(0);
+#pragma unroll
+        for (int t2 = 0; t2 < 2; ++t2) {
+            const RevTerm t = rev_of(C, t2);
+            const int a = t.axis, o = t.out;
+            if (g.n[a] == 1 || !((ACTIVE >> o) & 1)) continue;
+            T at[N], up[N];
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                const T above = a == 0 ? (k == N - 1 ? ux[o] : u[o].v[k == N - 1 ? k : k + 1]) : a == 1 ? uy[o].v[k] : uz[o].v[k];
+                at[k] = t.sign > 0 ? u[o].v[k] : -u[o].v[k];
+                up[k] = t.sign > 0 ? above : -above;
             }
-            const T *mt = g.metric[1][a];
-            auto dh = [&](T h, int cc) -> T {
-                const T dst = -g.cn * h;
-                const T v = t.sign > 0 ? dst : -dst;
-                return mt != nullptr ? v * mt[cc] : v;
-            };
-            contrib = contrib + dh(hm[C][k], c - 1);      // src[c] += D(c-1)
-            contrib = contrib - dh(hc[t.out], c);         // src[c] -= D(c)
-        }
-        e[C] = eb[C] + contrib;
-        T acc = T(0);
+            const T *old = A.pEb[q][a][t.j];
+            T *out = A.pEb[q ^ 1][a][t.j];
+            if (a == 0) {
+                if (last && g.periodic[0]) {             // the last cell's +1 neighbour is the row's first
+                    const T first = t.sign > 0 ? ux[o] : -ux[o];
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const Term t = term_of(C, k);
-            const int a = t.axis, c = co[a];
-            const T *mt = g.metric[0][a];
-            T d = sc[t.in] - smv[C][k];
-            if (mt != nullptr) d = d * mt[c];
-            if (((GEN >> a) & 1) && A.sPsiE[a][t.j] >= 0) {
-                const int r = adj_slab_row(A.slab[0][a], c);
-                if (r >= 0) {
-                    const long long p = g.psi_index(a, x, y, z, r, g.rows[0][a]);
-                    const T mem = slot[A.sPsiE[a][t.j] + p] * g.cb[0][a][c] + g.cc[0][a][c] * d;
-                    d = d * g.ck[0][a][c] + mem;
+                    for (int k = 0; k < N; ++k)
+                        if (x + k == nx - 1) up[k] = first;
+                }
+#pragma unroll
+                for (int k = 0; k < N; ++k) {
+                    const int c = x + k;
+                    if (XS) {
+                        if (c >= 1) at[k] = adj_slab_x_apply<T, 0>(A, c, y, z, old, out, true, at[k]);
+                        if (c + 1 <= nx - 1) up[k] = adj_slab_x_apply<T, 0>(A, c + 1, y, z, old, out, false, up[k]);
+                    }
+                    if (metric && c < nx) {
+                        at[k] = at[k] * mt(0, c);
+                        up[k] = up[k] * mt(0, c + 1 <= nx - 1 ? c + 1 : 0);
+                    }
+                    const bool wrap = g.periodic[0];
+                    if (c >= 1 || k > 0) contrib[k] = contrib[k] + at[k];
+                    if (!last || c + 1 <= nx - 1) contrib[k] = contrib[k] - up[k];
+                    if (k == 0 && x == 0 && wrap) contrib[k] = contrib[k] + at[k];
+                    if (last && c == nx - 1 && wrap) contrib[k] = contrib[k] - up[k];
+                }
+            } else {
+                const int c = a == 1 ? y : z, n = g.n[a];
+                if (c >= 1 && old != nullptr) {
+                    const int r = adj_slab_row(A.slab[0][a], c);
+                    if (r >= 0) {
+                        if (a == 1) adj_slab_row_apply<T, 0, 1>(A, r, x, y, z, old, out, true, at);
+                        else adj_slab_row_apply<T, 0, 2>(A, r, x, y, z, old, out, true, at);
+                    }
+                }
+                if (c + 1 <= n - 1 && old != nullptr) {
+                    const int r = adj_slab_row(A.slab[0][a], c + 1);
+                    if (r >= 0) {
+                        if (a == 1) adj_slab_row_apply<T, 0, 1>(A, r, x, y + 1, z, old, out, false, up);
+                        else adj_slab_row_apply<T, 0, 2>(A, r, x, y, z + 1, old, out, false, up);
+                    }
+                }
+                const T ma = metric ? mt(a, c) : T(1), mu = metric ? mt(a, c + 1 <= n - 1 ? c + 1 : 0) : T(1);
+                const bool wrap = g.periodic[a];
+#pragma unroll
+                for (int k = 0; k < N; ++k) {
+                    if (metric) {
+                        at[k] = at[k] * ma;
+                        up[k] = up[k] * mu;
+                    }
+                    if (c >= 1) contrib[k] = contrib[k] + at[k];
+                    if (c + 1 <= n - 1) contrib[k] = contrib[k] - up[k];
+                    if (wrap && c == 0) contrib[k] = contrib[k] + at[k];
+                    if (wrap && c == n - 1) contrib[k] = contrib[k] - up[k];
                 }
             }
-            acc = acc + (t.sign > 0 ? d : -d);
         }
-        s[C] = S0[C] + e[C] * acc;
-    }
+        Pack<T> r;
 #pragma unroll
-    for (int C = 0; C < 3; ++C) {
-        A.eb[q ^ 1][C][i] = e[C];
-        A.S[C][i] = s[C];
+        for (int k = 0; k < N; ++k) r.v[k] = x + k < nx ? hb[C].v[k] + contrib[k] : T(0);
+        pack_store(A.hb[q ^ 1][C] + i, r);
     }
 }
 
-// h_bar_new of the three components of a cell of a fast-path block; e_own: the cell's e_bar_new.
-template <typename T, int GEN>
-__device__ __forceinline__ void adj_h_fast(const AdjArgs<T> &A, int q, int x, int y, int z, long long i, const T *e_own) {
-    const Grid<T> &g = A.g;
-    const int co[3] = {x, y, z};
-    T ep[3][2], ie0[3], iep[3][2], hb[3];
-#pragma unroll
-    for (int o = 0; o < 3; ++o) {
-        ie0[o] = __ldg(g.inv_eps[o] + i);
-        hb[o] = __ldg(A.hb[q][o] + i);
-    }
-#pragma unroll
-    for (int C = 0; C < 3; ++C)
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const RevTerm t = rev_of(C, k);
-            ep[C][k] = __ldg(A.eb[q ^ 1][t.out] + i + g.stride(t.axis));
-            if (!((GEN >> t.axis) & 1)) iep[C][k] = __ldg(g.inv_eps[t.out] + i + g.stride(t.axis));
-        }
-    T out[3];
-#pragma unroll
-    for (int C = 0; C < 3; ++C) {
-        T contrib = T(0);
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const RevTerm t = rev_of(C, k);
-            const int a = t.axis, c = co[a];
-            if ((GEN >> a) & 1) {
-                const int xp = a == 0 ? x + 1 : x, yp = a == 1 ? y + 1 : y, zp = a == 2 ? z + 1 : z;
-                contrib = contrib + d_e(A, q, t, x, y, z, i, e_own[t.out], true);                   // src[c] += D(c)
-                contrib = contrib - d_e(A, q, t, xp, yp, zp, i + g.stride(a), ep[C][k], false);    // src[c] -= D(c+1)
-                continue;
-            }
-            const T *mt = g.metric[0][a];
-            auto de = [&](T ie, int cc, T eb) -> T {
-                const T dst = (g.cn * ie) * eb;
-                const T v = t.sign > 0 ? dst : -dst;
-                return mt != nullptr ? v * mt[cc] : v;
-            };
-            contrib = contrib + de(ie0[t.out], c, e_own[t.out]);       // src[c] += D(c)
-            contrib = contrib - de(iep[C][k], c + 1, ep[C][k]);        // src[c] -= D(c+1)
-        }
-        out[C] = hb[C] + contrib;
-    }
-#pragma unroll
-    for (int C = 0; C < 3; ++C) A.hb[q ^ 1][C][i] = out[C];
-}
-
-// Part 1 of the reverse step: e_bar_new of the own cell, and S += e_bar_new * curl_b(H_n).
+// Blocks of kPassThreads groups of one plane (blockIdx.x; plain groups first, then those near an x slab), planes on
+// blockIdx.y: ascending in the E pass, descending in the H pass. Reads parity q, writes q^1.
 template <typename T, int ACTIVE>
-__global__ void __launch_bounds__(kAdjX * kAdjY) k_adjoint_e(const __grid_constant__ AdjArgs<T> A, const T *__restrict__ slot, int q,
-                                                             int xs, int ys, int fast) {
-    const Grid<T> &g = A.g;
-    const int x0 = blockIdx.x * kAdjX - xs, y0 = blockIdx.y * kAdjY - ys;
-    const int x = x0 + threadIdx.x;
-    const int y = y0 + threadIdx.y;
-    const int z = blockIdx.z;
-    if (x < 0 || y < 0 || x >= g.n[0] || y >= g.n[1]) return;
-    const long long i = (long long)z * g.plane + (long long)y * g.pitch + x;
-    if (ACTIVE == 63 && fast && g.active == 63) {
-        switch (adj_class(A, x0, y0, z, true, 0)) {
-            case 0: adj_e_fast<T, 0>(A, slot, q, x, y, z, i); return;
-            case 1: adj_e_fast<T, 1>(A, slot, q, x, y, z, i); return;
-            case 2: adj_e_fast<T, 2>(A, slot, q, x, y, z, i); return;
-            case 3: adj_e_fast<T, 3>(A, slot, q, x, y, z, i); return;
-            case 4: adj_e_fast<T, 4>(A, slot, q, x, y, z, i); return;
-            case 5: adj_e_fast<T, 5>(A, slot, q, x, y, z, i); return;
-            case 6: adj_e_fast<T, 6>(A, slot, q, x, y, z, i); return;
-            case 7: adj_e_fast<T, 7>(A, slot, q, x, y, z, i); return;
-            default: break;
-        }
-    }
-    if (ACTIVE & 1) {
-        const T e = ebar_value<T, 0>(A, q, x, y, z, i, true);
-        A.eb[q ^ 1][0][i] = e;
-        A.S[0][i] = A.S[0][i] + e * forward_curl<T, 0>(A, slot, x, y, z, i);
-    }
-    if (ACTIVE & 2) {
-        const T e = ebar_value<T, 1>(A, q, x, y, z, i, true);
-        A.eb[q ^ 1][1][i] = e;
-        A.S[1][i] = A.S[1][i] + e * forward_curl<T, 1>(A, slot, x, y, z, i);
-    }
-    if (ACTIVE & 4) {
-        const T e = ebar_value<T, 2>(A, q, x, y, z, i, true);
-        A.eb[q ^ 1][2][i] = e;
-        A.S[2][i] = A.S[2][i] + e * forward_curl<T, 2>(A, slot, x, y, z, i);
+__global__ void __launch_bounds__(kPassThreads, 2) k_adjoint_e(const __grid_constant__ AdjArgs<T> A, const T *__restrict__ slot, int q) {
+    const unsigned p = blockIdx.x * kPassThreads + threadIdx.x;
+    if (p >= A.split.total) return;
+    const bool slab = p >= A.split.plain_total;
+    for (int z = blockIdx.y; z < A.g.n[2]; z += gridDim.y) {
+        const PassCell<long long> w = pass_cell<long long>(A.g, A.split, p, z, slab);
+        if (slab) adj_pass_e<T, ACTIVE, true>(A, slot, q, w);
+        else adj_pass_e<T, ACTIVE, false>(A, slot, q, w);
     }
 }
 
-// Part 2: h_bar_new of the own cell from the e_bar_new that part 1 stored (own cell and +x/+y/+z).
 template <typename T, int ACTIVE>
-__global__ void __launch_bounds__(kAdjX * kAdjY) k_adjoint_h(const __grid_constant__ AdjArgs<T> A, int q, int xs, int ys, int fast) {
-    const Grid<T> &g = A.g;
-    const int x0 = blockIdx.x * kAdjX - xs, y0 = blockIdx.y * kAdjY - ys;
-    const int x = x0 + threadIdx.x;
-    const int y = y0 + threadIdx.y;
-    const int z = blockIdx.z;
-    if (x < 0 || y < 0 || x >= g.n[0] || y >= g.n[1]) return;
-    const long long i = (long long)z * g.plane + (long long)y * g.pitch + x;
-    T e[3] = {T(0), T(0), T(0)};
-    if (ACTIVE & 1) e[0] = A.eb[q ^ 1][0][i];
-    if (ACTIVE & 2) e[1] = A.eb[q ^ 1][1][i];
-    if (ACTIVE & 4) e[2] = A.eb[q ^ 1][2][i];
-    if (ACTIVE == 63 && fast && g.active == 63) {
-        switch (adj_class(A, x0, y0, z, false, 1)) {
-            case 0: adj_h_fast<T, 0>(A, q, x, y, z, i, e); return;
-            case 1: adj_h_fast<T, 1>(A, q, x, y, z, i, e); return;
-            case 2: adj_h_fast<T, 2>(A, q, x, y, z, i, e); return;
-            case 3: adj_h_fast<T, 3>(A, q, x, y, z, i, e); return;
-            case 4: adj_h_fast<T, 4>(A, q, x, y, z, i, e); return;
-            case 5: adj_h_fast<T, 5>(A, q, x, y, z, i, e); return;
-            case 6: adj_h_fast<T, 6>(A, q, x, y, z, i, e); return;
-            case 7: adj_h_fast<T, 7>(A, q, x, y, z, i, e); return;
-            default: break;
-        }
+__global__ void __launch_bounds__(kPassThreads, 2) k_adjoint_h(const __grid_constant__ AdjArgs<T> A, int q) {
+    const unsigned p = blockIdx.x * kPassThreads + threadIdx.x;
+    if (p >= A.split.total) return;
+    const bool slab = p >= A.split.plain_total;
+    for (int z = A.g.n[2] - 1 - (int)blockIdx.y; z >= 0; z -= gridDim.y) {
+        const PassCell<long long> w = pass_cell<long long>(A.g, A.split, p, z, slab);
+        if (slab) adj_pass_h<T, ACTIVE, true>(A, q, w);
+        else adj_pass_h<T, ACTIVE, false>(A, q, w);
     }
-    if (ACTIVE & 8) A.hb[q ^ 1][0][i] = hbar_value<T, 0, true>(A, q, x, y, z, i, e);
-    if (ACTIVE & 16) A.hb[q ^ 1][1][i] = hbar_value<T, 1, true>(A, q, x, y, z, i, e);
-    if (ACTIVE & 32) A.hb[q ^ 1][2][i] = hbar_value<T, 2, true>(A, q, x, y, z, i, e);
 }
 
 // Observation seeds of one step: bar[family][comp][offset] += seed[k] (observers are distinct cells).

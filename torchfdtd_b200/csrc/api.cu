@@ -106,6 +106,7 @@ struct Layout {
     std::vector<TfsfLayout> tfsf;
     std::vector<AdeLayout> ade;
     size_t ade_map = 0;            // 3 x count int32 sample indices
+    size_t ade_at = 0;             // int64 element of each sample
     size_t volume[3];              // diagnostics cell volumes per axis (double), 0: unit
     size_t counter = 0, done = 0, status = 0, diag = 0, stage = 0;
     size_t grid_bar = 0;           // persistent stepping: arrival count and generation
@@ -428,6 +429,9 @@ void compute_layout(const tfd_desc *d, Layout &L) {
     for (int a = 0; a < 3; ++a) L.volume[a] = d->volume[a] ? b.take((size_t)n[a] * sizeof(double)) : 0;
     L.ade.resize(d->n_ade);
     L.ade_map = d->n_ade > 0 ? b.take((size_t)3 * L.count * sizeof(int)) : 0;
+    size_t samples = 0;
+    for (int k = 0; k < d->n_ade; ++k) samples += d->ade[k].samples;
+    L.ade_at = d->n_ade > 0 ? b.take(std::max<size_t>(1, samples) * sizeof(long long)) : 0;
     for (int k = 0; k < d->n_ade; ++k) {
         const tfd_ade &m = d->ade[k];
         L.ade[k].state = b.take(std::max<size_t>(1, (size_t)2 * m.poles * m.samples) * L.elem);
@@ -660,6 +664,8 @@ int create_typed(tfd_plan *p, const tfd_desc *d, cudaStream_t s) {
     // dispersive materials: the per-component sample map, pole coefficients, states (zeroed by zero_state)
     g.n_ade = d->n_ade;
     for (int c = 0; c < 3; ++c) g.ade_map[c] = nullptr;
+    g.ade_at = nullptr;
+    g.ade_samples = 0;
     if (d->n_ade > 0) {
         std::vector<int> map((size_t)3 * L.count, -1);
         int start = 0;
@@ -697,13 +703,43 @@ int create_typed(tfd_plan *p, const tfd_desc *d, cudaStream_t s) {
             st.k = cp + 2 * m.poles;
             st.P = p->ptr<T>(L.ade[k].state);
             st.Q = st.P + (size_t)m.poles * m.samples;
+        }
+        // Renumber the samples of each state in memory order (component, z, y, x): consecutive cells of a row hold
+        // consecutive pole states. The caller's order (z fastest) scattered a row's states over 32-byte sectors.
+        std::vector<int> renumbered(start), next(d->n_ade, 0);
+        std::vector<long long> at(start);
+        for (size_t e = 0; e < map.size(); ++e) {
+            if (map[e] < 0) continue;
+            int k = 0;
+            while (k + 1 < d->n_ade && map[e] >= g.ade[k + 1].start) ++k;
+            const int to = g.ade[k].start + next[k]++;
+            renumbered[map[e]] = to;
+            map[e] = to;
+            at[to] = (long long)e;
+        }
+        for (int k = 0; k < d->n_ade; ++k)
             if (L.ade[k].weight) {
-                std::vector<double> w(m.weight, m.weight + m.samples);
+                std::vector<double> w(d->ade[k].samples);
+                for (int j = 0; j < d->ade[k].samples; ++j) w[renumbered[g.ade[k].start + j] - g.ade[k].start] = d->ade[k].weight[j];
                 if (int rc = upload(s, p, L.ade[k].weight, w)) return rc;
             }
+        // The sample map is read only where a soft E source drives a dispersive sample.
+        bool driven = false;
+        for (int t = 0; t < d->n_sources && !driven; ++t) {
+            const tfd_source_term &q = d->sources[t];
+            if (q.family != 0) continue;
+            for (int z = q.lo[2]; z < q.hi[2] && !driven; ++z)
+                for (int y = q.lo[1]; y < q.hi[1] && !driven; ++y)
+                    for (int x = q.lo[0]; x < q.hi[0] && !driven; ++x)
+                        driven = map[(size_t)q.component * L.count + (size_t)z * g.plane + (size_t)y * L.pitch + x] >= 0;
         }
-        if (int rc = upload(s, p, L.ade_map, map)) return rc;
-        for (int c = 0; c < 3; ++c) g.ade_map[c] = p->ptr<int>(L.ade_map) + (size_t)c * L.count;
+        if (int rc = upload(s, p, L.ade_at, at)) return rc;
+        g.ade_at = p->ptr<long long>(L.ade_at);
+        g.ade_samples = start;
+        if (driven) {
+            if (int rc = upload(s, p, L.ade_map, map)) return rc;
+            for (int c = 0; c < 3; ++c) g.ade_map[c] = p->ptr<int>(L.ade_map) + (size_t)c * L.count;
+        }
     }
     // nonuniform-mesh factors
     for (int f = 0; f < 2; ++f)
@@ -1595,6 +1631,31 @@ bool two_pass_3d(const tfd_plan *p) {
     return d.precision == 8 || p->march_metric || seams || (long long)d.nx * d.ny * d.nz < kMarchMinCells;
 }
 
+// The groups of a row apart from the x slabs of family f (f < 0: of both), widened by `reach` cells.
+template <typename T>
+PassSplit pass_split(const tfd_plan *p, int f, int reach) {
+    constexpr int N = Pack<T>::N;
+    const int nx = p->desc.nx, groups = (nx + N - 1) / N;
+    std::vector<char> slab(groups, 0);
+    for (size_t q = 0; q < p->seg_f.size(); ++q)
+        if ((f < 0 || p->seg_f[q] == f) && p->seg_a[q] == 0)
+            for (int x = std::max(0, p->seg_lo[q] - reach); x < std::min(nx, p->seg_hi[q] + reach); ++x) slab[x / N] = 1;
+    PassSplit sp{};
+    for (int x = 0; x < groups; ++x) {                   // the longest run of groups clear of the slabs
+        int e = x;
+        while (e < groups && !slab[e]) ++e;
+        if (e - x > sp.plain) { sp.x_lo = x; sp.plain = e - x; }
+        x = std::max(x, e);
+    }
+    auto magic = [](int d) { return d <= 1 ? 0xffffffffu : (unsigned)(((1ull << 32) + d - 1) / d); };
+    sp.slab = groups - sp.plain;
+    sp.magic_plain = magic(sp.plain);
+    sp.magic_slab = magic(sp.slab);
+    sp.plain_total = (unsigned)sp.plain * p->desc.ny;
+    sp.total = (unsigned)groups * p->desc.ny;
+    return sp;
+}
+
 // The two-pass step's arguments: the grid, its slab bounds (or, with more than two slabs on an axis, the row
 // tables) and the 16-byte groups of a row.
 template <typename T>
@@ -1605,32 +1666,7 @@ int setup_pass(tfd_plan *p) {
     int count[2][3] = {};
     for (size_t q = 0; q < p->seg_f.size(); ++q) a.tables |= ++count[p->seg_f[q]][p->seg_a[q]] > 2;
     if (!a.tables) TFD_CHECK(slab_bounds(p, a.slab));
-    constexpr int N = Pack<T>::N;
-    const int groups = (a.g.n[0] + N - 1) / N;
-    auto magic = [](int d) { return d <= 1 ? 0xffffffffu : (unsigned)(((1ull << 32) + d - 1) / d); };
-    for (int f = 0; f < 2; ++f) {
-        // The longest run of groups that meet no x slab is the plain one.
-        std::vector<char> slab(groups, 0);
-        for (size_t q = 0; q < p->seg_f.size(); ++q)
-            if (p->seg_f[q] == f && p->seg_a[q] == 0)
-                for (int x = p->seg_lo[q]; x < p->seg_hi[q]; ++x) slab[x / N] = 1;
-        int from = 0, len = 0;
-        for (int x = 0; x < groups; ++x) {
-            int e = x;
-            while (e < groups && !slab[e]) ++e;
-            if (e - x > len) { from = x; len = e - x; }
-            x = std::max(x, e);
-        }
-        auto &sp = a.split[f];
-        sp.plain = len;
-        sp.x_lo = from;
-        sp.groups = groups;
-        sp.slab = groups - len;
-        sp.magic_plain = magic(sp.plain);
-        sp.magic_slab = magic(sp.slab);
-        sp.plain_total = (unsigned)sp.plain * a.g.n[1];
-        sp.total = (unsigned)groups * a.g.n[1];
-    }
+    for (int f = 0; f < 2; ++f) a.split[f] = pass_split<T>(p, f, 0);
     p->pass_metric = false;
     for (int f = 0; f < 2; ++f)
         for (int ax = 0; ax < 3; ++ax) {
@@ -1646,7 +1682,7 @@ template <typename T, int ACTIVE>
 void launch_pass_active(tfd_plan *p, bool h, cudaStream_t s) {
     const PassArgs<T> &a = p->pass<T>();
     const dim3 grid((a.split[0].total + kPassThreads - 1) / kPassThreads, (unsigned)std::min(a.g.n[2], 65535));
-    const bool ade = a.g.n_ade > 0;
+    const bool ade = a.g.ade_map[0] != nullptr;          // soft sources on dispersive samples
     if (p->pass_wide) {
         if (h) k_pass_h<T, ACTIVE, true, long long><<<grid, kPassThreads, 0, s>>>(a);
         else k_pass_e<T, ACTIVE, true, true, long long><<<grid, kPassThreads, 0, s>>>(a);
@@ -1792,11 +1828,13 @@ int launch_persist2d(tfd_plan *p, int nsteps, cudaStream_t s) {
     return TFD_OK;
 }
 
-// One two-pass step: the E pass, the TFSF boxes' E half step and E corrections, the H pass, the H half step and H
+// One two-pass step: the E pass, the dispersive samples, the TFSF boxes' E half step and E corrections, the H pass, the H half step and H
 // corrections (the observation launch follows in step_t).
 template <typename T>
 int launch_two_pass(tfd_plan *p, cudaStream_t s) {
     launch_pass<T>(p, false, s);
+    const int samples = p->grid<T>().ade_samples;
+    if (samples > 0) k_pass_ade<T><<<(samples + kPassThreads - 1) / kPassThreads, kPassThreads, 0, s>>>(p->pass<T>().g, samples);
     if (p->desc.n_tfsf == 0) {
         launch_pass<T>(p, true, s);
         return TFD_OK;
@@ -2169,7 +2207,8 @@ int tfd_step_launches(const tfd_plan *p, int32_t nsteps, int64_t *launches) {
         *launches = nsteps > 0 ? 1 : 0;
         return TFD_OK;
     }
-    long long per_step = p->desc.n_tfsf > 0 ? 5 : 3;         // two passes: E, (TFSF E), H, (TFSF H), observation
+    // Two passes: E, (dispersive samples), (TFSF E), H, (TFSF H), observation.
+    long long per_step = (p->desc.n_tfsf > 0 ? 5 : 3) + ((p->desc.precision == 8 ? p->gd.ade_samples : p->gf.ade_samples) > 0);
     if (!p->two_pass && p->kernel == TFD_KERNEL_TILE2D) {
         if ((p->persist_ctas > 0 || p->cluster2d.ranks > 0) && !p->in_batch) {
             *launches = nsteps > 0 ? 1 : 0;
@@ -2582,6 +2621,7 @@ int adjoint_create_t(tfd_adjoint *adj, cudaStream_t s) {
     for (int a = 0; a < 3; ++a)
         for (int j = 0; j < 2; ++j) A.sPsiE[a][j] = m.sPsiE[a][j];
     if (int rc = slab_bounds(p, A.slab)) return rc;
+    A.split = pass_split<T>(p, -1, 1);
     if (A.g.n[2] > 65535) return fail(TFD_ERR_UNSUPPORTED, "the adjoint step launches one z plane per grid row: nz above 65535");
     adj->used = adjoint_layout<T>(p, &A, adj->arena);
     TFD_CUDA(cudaMemsetAsync(adj->arena, 0, adj->used, s));
@@ -2597,32 +2637,20 @@ int adjoint_step_t(tfd_adjoint *adj, const void *snapshot, const void *seeds, cu
     if (seeds && n_obs > 0)
         k_adjoint_seed<T><<<std::max(1, std::min(1184, (n_obs + 255) / 256)), 256, 0, s>>>(A, p->ptr<TraceDev>(p->L.trace_tab), n_obs,
                                                                                        (const T *)seeds, adj->q);
-    const Grid<T> &g = A.g;
-    // x tiles at multiples of 32 (rows aligned to 128 bytes: measured 13 % faster for k_adjoint_e than tiles
-    // starting at x = 1, which put one more column of tiles on the fast path); y tiles shifted to start at y = 1,
-    // so the first tile row holds the y = 0 face alone. A tile whose cells all lie in [1, n-2] takes the fast path.
-    const int exs = 0, eys = kAdjY - 1;
-    const int hxs = exs, hys = eys;
-    auto grid_of = [&](int xs, int ys) {
-        return dim3((unsigned)((g.n[0] + xs + kAdjX - 1) / kAdjX), (unsigned)((g.n[1] + ys + kAdjY - 1) / kAdjY), (unsigned)g.n[2]);
-    };
-    const dim3 ge = grid_of(exs, eys), gh = grid_of(hxs, hys);
-    const char *env = getenv("TFD_ADJ_FAST");
-    const int fast = (env && std::atoi(env) == 0) ? 0 : 1;
-    const dim3 block(kAdjX, kAdjY);
+    const dim3 grid((A.split.total + kPassThreads - 1) / kPassThreads, (unsigned)std::min(A.g.n[2], 65535));
     const T *slot = (const T *)snapshot;
     switch (p->desc.components) {
         case kMaskTM:
-            k_adjoint_e<T, kMaskTM><<<ge, block, 0, s>>>(A, slot, adj->q, exs, eys, fast);
-            k_adjoint_h<T, kMaskTM><<<gh, block, 0, s>>>(A, adj->q, hxs, hys, fast);
+            k_adjoint_e<T, kMaskTM><<<grid, kPassThreads, 0, s>>>(A, slot, adj->q);
+            k_adjoint_h<T, kMaskTM><<<grid, kPassThreads, 0, s>>>(A, adj->q);
             break;
         case kMaskTE:
-            k_adjoint_e<T, kMaskTE><<<ge, block, 0, s>>>(A, slot, adj->q, exs, eys, fast);
-            k_adjoint_h<T, kMaskTE><<<gh, block, 0, s>>>(A, adj->q, hxs, hys, fast);
+            k_adjoint_e<T, kMaskTE><<<grid, kPassThreads, 0, s>>>(A, slot, adj->q);
+            k_adjoint_h<T, kMaskTE><<<grid, kPassThreads, 0, s>>>(A, adj->q);
             break;
         default:
-            k_adjoint_e<T, kMaskAll><<<ge, block, 0, s>>>(A, slot, adj->q, exs, eys, fast);
-            k_adjoint_h<T, kMaskAll><<<gh, block, 0, s>>>(A, adj->q, hxs, hys, fast);
+            k_adjoint_e<T, kMaskAll><<<grid, kPassThreads, 0, s>>>(A, slot, adj->q);
+            k_adjoint_h<T, kMaskAll><<<grid, kPassThreads, 0, s>>>(A, adj->q);
             break;
     }
     TFD_CUDA(cudaGetLastError());

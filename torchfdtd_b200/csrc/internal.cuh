@@ -47,8 +47,8 @@ struct SourceTerm {
 constexpr int kMaxAde = 8;
 constexpr int kMaxPoles = 16;
 
-// One dispersive material state on the device: samples [start, start + samples) of the plan's sample list,
-// P and Q as [poles][samples], coefficients in the field precision.
+// One dispersive material state on the device: samples [start, start + samples) of the plan's sample list, numbered in
+// memory order (component, z, y, x), P and Q as [poles][samples], coefficients in the field precision.
 template <typename T>
 struct AdeDev {
     int start, samples, poles;
@@ -82,8 +82,11 @@ struct Grid {
     int n_src;
     SourceTerm src[kMaxSources];
     const T *src_values;         // [n_src][steps]
-    // Dispersive materials: per E component the sample index of each cell (-1: none); nullptr without any.
+    // Dispersive materials: each sample's element (component * count + element index), and per E component the sample
+    // index of each cell (-1: none; nullptr when no soft E source drives a dispersive sample: nothing else reads it).
     const int *ade_map[3];
+    const long long *ade_at;
+    int ade_samples;
     int n_ade;
     AdeDev<T> ade[kMaxAde];
     long long *counter;

@@ -36,15 +36,18 @@ constexpr int kPassThreads = 256;
 // 128 in FP64.
 template <typename T> constexpr int kPassBlocks = sizeof(T) == 4 ? 3 : 2;
 
+// Groups of a row: those that meet no x slab (`plain` of them from x_lo on) and those that do (the first x_lo and the last
+// ones). A plane's groups are walked plain ones first, then the slab ones, so that a warp holds one kind: with both in a
+// warp the slab path ran for every warp of a 256-cell row (786 instructions per warp and pass, 256^3 cells: 488 against
+// 290 us per step).
+struct PassSplit { int plain, x_lo, slab; unsigned magic_plain, magic_slab, plain_total, total; };
+
 template <typename T>
 struct PassArgs {
     Grid<T> g;
     int slab[2][3][4];           // per family and axis: lo0, hi0, lo1, hi1 of the two CPML slabs
     int tables;                  // 1: more than two slabs on some axis, slab rows come from the row tables
-    // Groups of a row, split by family: those that meet no x slab (from x_lo on) and those that do (the first x_lo
-    // and the last ones). A plane's groups are walked plain ones first, then the slab ones, so that a warp holds one
-    // kind: with both in a warp the slab path ran for every warp of a 256-cell row (786 instructions per warp).
-    struct Split { int plain, x_lo, slab, groups; unsigned magic_plain, magic_slab, plain_total, total; } split[2];
+    PassSplit split[2];          // per family
 };
 
 template <typename T> struct alignas(16) Pack { static constexpr int N = 16 / sizeof(T); T v[N]; };
@@ -136,28 +139,63 @@ __device__ __forceinline__ void pass_cpml(const PassArgs<T> &A, const PassCell<I
     pack_store(out + p, m);
 }
 
-// The coupled trapezoidal ADE of dispersive sample j: E_new from the free update and the old E, the pole states
-// advanced. Reference operation order (torchfdtd/materials.py:67-88).
+// Dispersive samples (threads j of total): the coupled trapezoidal ADE turns the free update that the E pass stored into
+// E_new and advances the pole states, then the soft sources of the cell are added (the E pass leaves dispersive samples
+// to this sweep). Reference operation order (torchfdtd/materials.py:67-88).
+//
+// A sweep of its own, one thread per sample in memory order, because the samples are a small share of the cells but touch
+// most warps: inside the E pass every warp that held one sample ran the whole correction for it (201 x 187 x 163 cells,
+// 1.2 M samples: 306 us per step, 164 with this sweep).
 template <typename T>
-__device__ __forceinline__ T ade_correct(const Grid<T> &g, int j, T old, T free) {
+__device__ __forceinline__ void pass_ade(const Grid<T> &g, int j, int par, long long n) {
+    const long long at = g.ade_at[j];
+    const int c = at >= 2 * g.count ? 2 : at >= g.count ? 1 : 0;
+    const long long i = at - c * g.count;
+    const T old = g.E[par][c][i], free = g.E[par ^ 1][c][i];
     int s = 0;
     while (s + 1 < g.n_ade && j >= g.ade[s + 1].start) ++s;
     const AdeDev<T> &st = g.ade[s];
     const int l = j - st.start, ns = st.samples;
-    auto response = [&](int p) -> T { return (st.Q[p * ns + l] - st.a[p] * st.P[p * ns + l]) / st.d[p]; };
-    T total = response(0);
-    for (int p = 1; p < st.poles; ++p) total = total + response(p);
-    const T e = (st.eps * free - st.ksum * old - total) / st.denom;
-    for (int p = 0; p < st.poles; ++p) {
-        const T delta = response(p) + st.k[p] * (e + old);
-        st.P[p * ns + l] = st.P[p * ns + l] + delta;
-        st.Q[p * ns + l] = -st.Q[p * ns + l] + T(2) * delta;
+    T e;
+    if (st.poles == 1) {
+        const T P = st.P[l], Q = st.Q[l];
+        const T response = (Q - st.a[0] * P) / st.d[0];
+        e = (st.eps * free - st.ksum * old - response) / st.denom;
+        const T delta = response + st.k[0] * (e + old);
+        st.P[l] = P + delta;
+        st.Q[l] = -Q + T(2) * delta;
+    } else {
+        auto response = [&](int p) -> T { return (st.Q[p * ns + l] - st.a[p] * st.P[p * ns + l]) / st.d[p]; };
+        T total = response(0);
+        for (int p = 1; p < st.poles; ++p) total = total + response(p);
+        e = (st.eps * free - st.ksum * old - total) / st.denom;
+        for (int p = 0; p < st.poles; ++p) {
+            const T delta = response(p) + st.k[p] * (e + old);
+            st.P[p * ns + l] = st.P[p * ns + l] + delta;
+            st.Q[p * ns + l] = -st.Q[p * ns + l] + T(2) * delta;
+        }
     }
-    return e;
+    if (g.n_src > 0) {
+        const int z = (int)(i / g.plane), y = (int)(i % g.plane) / g.pitch, x = (int)(i % g.plane) % g.pitch;
+        for (int t = 0; t < g.n_src; ++t) {
+            const SourceTerm &q = g.src[t];
+            if (q.family == 0 && q.comp == c && x >= q.lo[0] && x < q.hi[0] && y >= q.lo[1] && y < q.hi[1] && z >= q.lo[2] && z < q.hi[2])
+                e = e + g.src_values[(long long)t * g.steps + n];
+        }
+    }
+    g.E[par ^ 1][c][i] = e;
 }
 
-// Soft sources of a family over a group, one term after the other (ascending index).
-template <typename T, typename I>
+template <typename T>
+__global__ void __launch_bounds__(kPassThreads) k_pass_ade(const __grid_constant__ Grid<T> g, int samples) {
+    const long long n = *g.counter;
+    if (n >= g.steps) return;
+    const int j = blockIdx.x * kPassThreads + threadIdx.x;
+    if (j < samples) pass_ade(g, j, (int)(n & 1), n);
+}
+
+// Soft sources of a family over a group, one term after the other (ascending index). ADE: dispersive samples are left out.
+template <typename T, bool ADE, typename I>
 __device__ __forceinline__ void pass_sources(const Grid<T> &g, int family, long long n, const PassCell<I> &q, Pack<T> (&f)[3]) {
     constexpr int N = Pack<T>::N;
     for (int s = 0; s < g.n_src; ++s) {
@@ -169,7 +207,7 @@ __device__ __forceinline__ void pass_sources(const Grid<T> &g, int family, long 
         for (int c = 0; c < 3; ++c)
 #pragma unroll
             for (int k = 0; k < N; ++k)
-                if (t.comp == c && q.x + k >= t.lo[0] && q.x + k < t.hi[0]) f[c].v[k] = f[c].v[k] + v;
+                if (t.comp == c && q.x + k >= t.lo[0] && q.x + k < t.hi[0] && !(ADE && g.ade_map[c][q.i + k] >= 0)) f[c].v[k] = f[c].v[k] + v;
     }
 }
 
@@ -280,18 +318,8 @@ __device__ __forceinline__ void pass_e(const PassArgs<T> &A, const PassCell<I> &
         dy(hx, hx_y, 1, d1);
         update(2, false, true);
     }
-    if (ADE && g.n_ade > 0) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            if (!((ACTIVE >> c) & 1)) continue;
-#pragma unroll
-            for (int k = 0; k < N; ++k) {
-                const int j = q.x + k < g.n[0] ? g.ade_map[c][i + k] : -1;
-                if (j >= 0) e[c].v[k] = ade_correct(g, j, eo[c].v[k], e[c].v[k]);
-            }
-        }
-    }
-    pass_sources(g, 0, n, q, e);
+    if (ADE && g.ade_map[0] != nullptr) pass_sources<T, true>(g, 0, n, q, e);
+    else pass_sources<T, false>(g, 0, n, q, e);
     const bool tail = q.x + N > g.n[0];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -412,7 +440,7 @@ __device__ __forceinline__ void pass_h(const PassArgs<T> &A, const PassCell<I> &
         dy(ex, ex_y, 1, d1);
         update(2, false, true);
     }
-    pass_sources(g, 1, n, q, h);
+    pass_sources<T, false>(g, 1, n, q, h);
     const bool tail = q.x + N > nx;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -440,10 +468,9 @@ __device__ __forceinline__ int pass_divide(unsigned p, unsigned d, unsigned m, i
     return y;
 }
 
-// Group p of plane z in the order of a family's split; slab: whether it meets an x slab.
+// Group p of plane z in the order of a split; slab: whether it meets an x slab.
 template <typename I, typename T>
-__device__ __forceinline__ PassCell<I> pass_cell(const PassArgs<T> &A, int f, unsigned p, int z, bool slab) {
-    const auto &s = A.split[f];
+__device__ __forceinline__ PassCell<I> pass_cell(const Grid<T> &g, const PassSplit &s, unsigned p, int z, bool slab) {
     PassCell<I> q;
     int xg;
     if (!slab) {
@@ -455,7 +482,7 @@ __device__ __forceinline__ PassCell<I> pass_cell(const PassArgs<T> &A, int f, un
     }
     q.x = xg * Pack<T>::N;
     q.z = z;
-    q.i = (I)z * (I)A.g.plane + (I)q.y * A.g.pitch + q.x;
+    q.i = (I)z * (I)g.plane + (I)q.y * g.pitch + q.x;
     return q;
 }
 
@@ -464,7 +491,7 @@ template <typename T, int ACTIVE, bool METRIC, bool ADE, typename I>
 __device__ __forceinline__ void pass_block_e(const PassArgs<T> &A, unsigned p, int z, int par, long long n) {
     if (p >= A.split[0].total) return;
     const bool slab = p >= A.split[0].plain_total;
-    const PassCell<I> q = pass_cell<I>(A, 0, p, z, slab);
+    const PassCell<I> q = pass_cell<I>(A.g, A.split[0], p, z, slab);
     if (slab) pass_e<T, ACTIVE, METRIC, ADE, true>(A, q, par, n);
     else pass_e<T, ACTIVE, METRIC, ADE, false>(A, q, par, n);
 }
@@ -473,7 +500,7 @@ template <typename T, int ACTIVE, bool METRIC, typename I>
 __device__ __forceinline__ void pass_block_h(const PassArgs<T> &A, unsigned p, int z, int par, long long n) {
     if (p >= A.split[1].total) return;
     const bool slab = p >= A.split[1].plain_total;
-    const PassCell<I> q = pass_cell<I>(A, 1, p, z, slab);
+    const PassCell<I> q = pass_cell<I>(A.g, A.split[1], p, z, slab);
     if (slab) pass_h<T, ACTIVE, METRIC, true>(A, q, par, n);
     else pass_h<T, ACTIVE, METRIC, false>(A, q, par, n);
 }
@@ -552,6 +579,10 @@ __global__ void __launch_bounds__(kPassStepThreads, 1) k_pass_steps(const __grid
         for (int it = blockIdx.x; it < items; it += gridDim.x)
             pass_block_e<T, ACTIVE, METRIC, ADE, int>(A, (it % per_plane) * kPassStepThreads + threadIdx.x, it / per_plane, par, n);
         if (!barrier()) return;
+        if (ADE) {
+            for (int j = blockIdx.x * kPassStepThreads + threadIdx.x; j < g.ade_samples; j += gridDim.x * kPassStepThreads) pass_ade(g, j, par, n);
+            if (!barrier()) return;
+        }
         for (int it = blockIdx.x; it < items; it += gridDim.x)
             pass_block_h<T, ACTIVE, METRIC, int>(A, (it % per_plane) * kPassStepThreads + threadIdx.x, it / per_plane, par, n);
         if (!barrier()) return;
