@@ -306,6 +306,13 @@ int tfd_adjoint_bytes(tfd_plan *plan, size_t *bytes);
 int tfd_adjoint_create(tfd_plan *plan, void *arena, size_t arena_bytes, void *stream, tfd_adjoint **adjoint);
 int tfd_adjoint_reset(tfd_adjoint *adjoint, void *stream);
 int tfd_adjoint_step(tfd_adjoint *adjoint, const void *snapshot, const void *seeds, void *stream);
+/* A whole checkpoint segment in one call: restores `checkpoint` (the state before the segment's first step), replays the
+ * first count - 1 steps, each leaving what its successor's transpose reads in slot 1, 2, .. of `replay` (count slots of
+ * slot_bytes, at least tfd_state_bytes and a multiple of 256; slot 0 is not used, a slot is not a full restart state),
+ * then transposes the count steps in reverse with `seeds` (count rows of one value per trace, or null). The replayed
+ * steps record no traces or planes. Same result as load, save, step and tfd_adjoint_step one by one. */
+int tfd_adjoint_segment(tfd_adjoint *adjoint, const void *checkpoint, int32_t count, void *replay, size_t slot_bytes,
+                        const void *seeds, void *stream);
 /* S in the reference layout (nx, ny, nz, 3), one value per E component (zero for components 2D does not
  * advance); TFD_HOST or TFD_DEVICE destination. */
 int tfd_adjoint_sensitivity(tfd_adjoint *adjoint, void *dst, int where, void *stream);

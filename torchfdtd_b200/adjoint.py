@@ -10,7 +10,8 @@ checkpoints.
 
 Checkpointing is the two-level square-root scheme: the forward pass stores K restart snapshots (default
 K = ceil(sqrt(steps))) in device memory; the backward pass restores each segment's snapshot, replays the
-segment once while saving its states, and transposes the segment's steps in reverse from those states.
+segment once while saving what the transposes read, and transposes the segment's steps in reverse
+(``tfd_adjoint_segment``).
 Every forward step is therefore recomputed exactly once, and device memory holds about 2 sqrt(steps)
 restart states (the reference's binomial schedule, differentiable.py:644-652, trades more replays for
 fewer slots; on a 180 GB device the square-root schedule's memory is affordable and its replay count is
@@ -141,14 +142,9 @@ class _Engine:
         for k in range(self.slots - 1, -1, -1):
             start = k * self.segment
             end = min(start + self.segment, steps)
-            self.grid.load_state(self.checkpoints[k])
-            for j in range(end - start):
-                self.grid.save_state(self.replay[j])
-                if start + j + 1 < end:
-                    self.grid.step(1)
-                    replayed += 1
-            for n in range(end - 1, start - 1, -1):
-                self.adjoint.step(self.replay[n - start], seeds[n] if seeds.shape[1] else None)
+            # One call per segment: a call per step cost more host time than the 2D kernels run.
+            self.adjoint.segment(self.checkpoints[k], end - start, self.replay, seeds[start:end] if seeds.shape[1] else None)
+            replayed += end - start - 1
         S = self.adjoint.sensitivity()
         eps = epsilon.detach()
         if eps.ndim == 3:

@@ -60,6 +60,17 @@ __device__ __forceinline__ int adj_slab_row(const int *b, int c) {
     return (c >= b[0] && c < b[1]) ? c - b[0] : (c >= b[2] && c < b[3]) ? (b[1] - b[0]) + (c - b[2]) : -1;
 }
 
+// Loads through the read-only path: the memories and snapshots a reverse pass reads are not written by its launch, and
+// without it every load waits behind the stores before it, which could alias it for the compiler.
+__device__ __forceinline__ Pack<float> pack_ldg(const float *p) {
+    const float4 q = __ldg(reinterpret_cast<const float4 *>(p));
+    return Pack<float>{{q.x, q.y, q.z, q.w}};
+}
+__device__ __forceinline__ Pack<double> pack_ldg(const double *p) {
+    const double2 q = __ldg(reinterpret_cast<const double2 *>(p));
+    return Pack<double>{{q.x, q.y}};
+}
+
 // CPML transpose of the D values v[] of a group's cells in one y or z slab row r: m = psi_bar + v; psi_bar <- b m (when
 // own); v <- v / kappa + c m.
 template <typename T, int F, int a>
@@ -69,8 +80,8 @@ __device__ __forceinline__ void adj_slab_row_apply(const AdjArgs<T> &A, int r, i
     const Grid<T> &g = A.g;
     const int c = a == 1 ? y : z;
     const long long p = g.psi_index(a, x, y, z, r, g.rows[F][a]);
-    const T b = g.cb[F][a][c], cc = g.cc[F][a][c], ck = g.ck[F][a][c];
-    const Pack<T> m0 = pack_load(old + p);
+    const T b = __ldg(g.cb[F][a] + c), cc = __ldg(g.cc[F][a] + c), ck = __ldg(g.ck[F][a] + c);
+    const Pack<T> m0 = pack_ldg(old + p);
     Pack<T> w;
 #pragma unroll
     for (int k = 0; k < N; ++k) {
@@ -89,9 +100,9 @@ __device__ __forceinline__ T adj_slab_x_apply(const AdjArgs<T> &A, int x, int y,
     const int r = adj_slab_row(A.slab[F][0], x);
     if (r < 0) return v;
     const long long p = g.psi_index(0, x, y, z, r, g.rows[F][0]);
-    const T m = old[p] + v;
-    if (own) out[p] = g.cb[F][0][x] * m;
-    return v * g.ck[F][0][x] + g.cc[F][0][x] * m;
+    const T m = __ldg(old + p) + v;
+    if (own) out[p] = __ldg(g.cb[F][0] + x) * m;
+    return v * __ldg(g.ck[F][0] + x) + __ldg(g.cc[F][0] + x) * m;
 }
 
 // e_bar_new and the sensitivity of a group. XS: the group or a neighbour of its ends lies in an x slab.
@@ -115,14 +126,14 @@ __device__ __forceinline__ void adj_pass_e(const AdjArgs<T> &A, const T *__restr
         hx[c] = fx[c] = T(0);
         if ((ACTIVE >> (3 + c)) & 1) {
             const T *hb = A.hb[q][c], *sf = slot + A.sH[c];
-            h[c] = pack_load(hb + i);
-            f[c] = pack_load(sf + i);
-            if (c != 0) { hx[c] = hb[ix]; fx[c] = sf[ix]; }
-            if (c != 1 && ny > 1) { hy[c] = pack_load(hb + iy); fy[c] = pack_load(sf + iy); }
-            if (c != 2 && nz > 1) { hz[c] = pack_load(hb + iz); fz[c] = pack_load(sf + iz); }
+            h[c] = pack_ldg(hb + i);
+            f[c] = pack_ldg(sf + i);
+            if (c != 0) { hx[c] = __ldg(hb + ix); fx[c] = __ldg(sf + ix); }
+            if (c != 1 && ny > 1) { hy[c] = pack_ldg(hb + iy); fy[c] = pack_ldg(sf + iy); }
+            if (c != 2 && nz > 1) { hz[c] = pack_ldg(hb + iz); fz[c] = pack_ldg(sf + iz); }
         }
         if ((ACTIVE >> c) & 1) {
-            eb[c] = pack_load(A.eb[q][c] + i);
+            eb[c] = pack_ldg(A.eb[q][c] + i);
             S[c] = pack_load(A.S[c] + i);
         }
     }
@@ -233,15 +244,15 @@ __device__ __forceinline__ void adj_pass_e(const AdjArgs<T> &A, const T *__restr
                         for (int k = 0; k < N; ++k) {
                             const int c = x + k, r = c < nx ? adj_slab_row(A.slab[0][0], c) : -1;
                             if (c > 0 && r >= 0) {
-                                const T m = psi[g.psi_index(0, c, y, z, r, g.rows[0][0])] * g.cb[0][0][c] + g.cc[0][0][c] * d[k];
-                                d[k] = d[k] * g.ck[0][0][c] + m;
+                                const T m = __ldg(psi + g.psi_index(0, c, y, z, r, g.rows[0][0])) * __ldg(g.cb[0][0] + c) + __ldg(g.cc[0][0] + c) * d[k];
+                                d[k] = d[k] * __ldg(g.ck[0][0] + c) + m;
                             }
                         }
                 } else {
                     const int r = c0 > 0 ? adj_slab_row(A.slab[0][a], c0) : -1;
                     if (r >= 0) {
-                        const Pack<T> m0 = pack_load(psi + g.psi_index(a, x, y, z, r, g.rows[0][a]));
-                        const T b = g.cb[0][a][c0], cc = g.cc[0][a][c0], ck = g.ck[0][a][c0];
+                        const Pack<T> m0 = pack_ldg(psi + g.psi_index(a, x, y, z, r, g.rows[0][a]));
+                        const T b = __ldg(g.cb[0][a] + c0), cc = __ldg(g.cc[0][a] + c0), ck = __ldg(g.ck[0][a] + c0);
 #pragma unroll
                         for (int k = 0; k < N; ++k) {
                             const T m = m0.v[k] * b + cc * d[k];
@@ -294,12 +305,12 @@ __device__ __forceinline__ void adj_pass_h(const AdjArgs<T> &A, int q, const Pas
         ux[c] = T(0);
         if ((ACTIVE >> c) & 1) {
             const T *eb = A.eb[q ^ 1][c], *ie = g.inv_eps[c];
-            u[c] = scaled(pack_load(ie + i), pack_load(eb + i));
-            if (c != 0) ux[c] = (g.cn * ie[ix]) * eb[ix];
-            if (c != 1 && ny > 1) uy[c] = scaled(pack_load(ie + iy), pack_load(eb + iy));
-            if (c != 2 && nz > 1) uz[c] = scaled(pack_load(ie + iz), pack_load(eb + iz));
+            u[c] = scaled(pack_ldg(ie + i), pack_ldg(eb + i));
+            if (c != 0) ux[c] = (g.cn * __ldg(ie + ix)) * __ldg(eb + ix);
+            if (c != 1 && ny > 1) uy[c] = scaled(pack_ldg(ie + iy), pack_ldg(eb + iy));
+            if (c != 2 && nz > 1) uz[c] = scaled(pack_ldg(ie + iz), pack_ldg(eb + iz));
         }
-        if ((ACTIVE >> (3 + c)) & 1) hb[c] = pack_load(A.hb[q][c] + i);
+        if ((ACTIVE >> (3 + c)) & 1) hb[c] = pack_ldg(A.hb[q][c] + i);
     }
     const bool metric = g.metric[0][0] != nullptr || g.metric[0][1] != nullptr || g.metric[0][2] != nullptr;
     auto mt = [&](int a, int c) -> T { return g.metric[0][a] != nullptr ? g.metric[0][a][c] : T(1); };

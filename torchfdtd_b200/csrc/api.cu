@@ -1604,10 +1604,9 @@ int setup_pass_steps(tfd_plan *p) {
 }
 
 template <typename T>
-int launch_pass_steps(tfd_plan *p, int nsteps, cudaStream_t s) {
-    const PassArgs<T> &a = p->pass<T>();
+int launch_pass_steps(tfd_plan *p, const PassArgs<T> &a, int nsteps, bool observe, cudaStream_t s) {
     const MonitorArgs<T> m = monitor_args<T>(p);
-    const int mgx = std::max(1, (p->max_samples + kPassStepThreads - 1) / kPassStepThreads), mgy = std::max(1, p->desc.n_planes);
+    const int mgx = observe ? std::max(1, (p->max_samples + kPassStepThreads - 1) / kPassStepThreads) : 0, mgy = std::max(1, p->desc.n_planes);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr;
     pass_steps_config(cfg, attr, p->pass_cluster, p->pass_ctas, s);
@@ -1679,8 +1678,7 @@ int setup_pass(tfd_plan *p) {
 // One pass (E, or H from the stored E_new) of the two-pass step. Arrays of 2^31 elements and more take the variant with
 // 64-bit indices, which handles every other feature at run time.
 template <typename T, int ACTIVE>
-void launch_pass_active(tfd_plan *p, bool h, cudaStream_t s) {
-    const PassArgs<T> &a = p->pass<T>();
+void launch_pass_active(tfd_plan *p, const PassArgs<T> &a, bool h, cudaStream_t s) {
     const dim3 grid((a.split[0].total + kPassThreads - 1) / kPassThreads, (unsigned)std::min(a.g.n[2], 65535));
     const bool ade = a.g.ade_map[0] != nullptr;          // soft sources on dispersive samples
     if (p->pass_wide) {
@@ -1699,11 +1697,11 @@ void launch_pass_active(tfd_plan *p, bool h, cudaStream_t s) {
 }
 
 template <typename T>
-void launch_pass(tfd_plan *p, bool h, cudaStream_t s) {
+void launch_pass(tfd_plan *p, const PassArgs<T> &a, bool h, cudaStream_t s) {
     switch (p->grid<T>().active) {
-        case kMaskTM: launch_pass_active<T, kMaskTM>(p, h, s); break;
-        case kMaskTE: launch_pass_active<T, kMaskTE>(p, h, s); break;
-        default: launch_pass_active<T, kMaskAll>(p, h, s); break;
+        case kMaskTM: launch_pass_active<T, kMaskTM>(p, a, h, s); break;
+        case kMaskTE: launch_pass_active<T, kMaskTE>(p, a, h, s); break;
+        default: launch_pass_active<T, kMaskAll>(p, a, h, s); break;
     }
 }
 
@@ -1831,12 +1829,12 @@ int launch_persist2d(tfd_plan *p, int nsteps, cudaStream_t s) {
 // One two-pass step: the E pass, the dispersive samples, the TFSF boxes' E half step and E corrections, the H pass, the H half step and H
 // corrections (the observation launch follows in step_t).
 template <typename T>
-int launch_two_pass(tfd_plan *p, cudaStream_t s) {
-    launch_pass<T>(p, false, s);
+int launch_two_pass(tfd_plan *p, const PassArgs<T> &pass, cudaStream_t s) {
+    launch_pass<T>(p, pass, false, s);
     const int samples = p->grid<T>().ade_samples;
     if (samples > 0) k_pass_ade<T><<<(samples + kPassThreads - 1) / kPassThreads, kPassThreads, 0, s>>>(p->pass<T>().g, samples);
     if (p->desc.n_tfsf == 0) {
-        launch_pass<T>(p, true, s);
+        launch_pass<T>(p, pass, true, s);
         return TFD_OK;
     }
     const Grid<T> &g = p->grid<T>();
@@ -1851,7 +1849,7 @@ int launch_two_pass(tfd_plan *p, cudaStream_t s) {
     for (int k = 0; k < a.boxes; ++k) longest = std::max(longest, a.box[k].count + std::max(a.box[k].n[0], a.box[k].n[1]));
     const dim3 tgrid((unsigned)((longest + kTfsfThreads - 1) / kTfsfThreads), (unsigned)a.boxes);
     k_tfsf<T><<<tgrid, kTfsfThreads, 0, s>>>(a, 0);
-    launch_pass<T>(p, true, s);
+    launch_pass<T>(p, pass, true, s);
     k_tfsf<T><<<tgrid, kTfsfThreads, 0, s>>>(a, 1);
     return TFD_OK;
 }
@@ -1867,14 +1865,14 @@ int step_t(tfd_plan *p, int nsteps, cudaStream_t s) {
         return TFD_OK;
     }
     if (p->two_pass && p->pass_ctas > 0) {
-        if (nsteps > 0) TFD_CHECK(launch_pass_steps<T>(p, nsteps, s));
+        if (nsteps > 0) TFD_CHECK(launch_pass_steps<T>(p, p->pass<T>(), nsteps, true, s));
         return TFD_OK;
     }
     const MonitorArgs<T> m = monitor_args<T>(p);
     dim3 mgrid((unsigned)std::max(1, (p->max_samples + kMonitorThreads - 1) / kMonitorThreads), (unsigned)std::max(1, p->desc.n_planes));
     for (int k = 0; k < nsteps; ++k) {
         if (p->two_pass) {
-            TFD_CHECK(launch_two_pass<T>(p, s));
+            TFD_CHECK(launch_two_pass<T>(p, p->pass<T>(), s));
         } else if (p->kernel == TFD_KERNEL_MARCH) {
             launch_march_any<T>(p, s);
         } else {
@@ -2544,7 +2542,14 @@ __global__ void k_state_copy(const __grid_constant__ StateCopy<T> sc, char *slot
     const int par = (int)(n & 1);
     T *arr = sc.a[k][par];
     T *snap = (T *)slot + sc.off[k];
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < sc.len[k]; e += (long long)gridDim.x * blockDim.x) {
+    // 16 bytes at a time (every array of a plan and a snapshot starts on a 256-byte boundary), then the remainder.
+    constexpr int N = 16 / sizeof(T);
+    const uint4 *from = reinterpret_cast<const uint4 *>(save ? arr : snap);
+    uint4 *to = reinterpret_cast<uint4 *>(save ? snap : arr);
+    const long long packs = sc.len[k] / N, first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    for (long long e = first; e < packs; e += (long long)gridDim.x * blockDim.x) to[e] = from[e];
+    if (first < sc.len[k] - packs * N) {
+        const long long e = packs * N + first;
         if (save) snap[e] = arr[e];
         else arr[e] = snap[e];
     }
@@ -2561,7 +2566,7 @@ int state_copy_t(tfd_plan *p, char *slot, bool save, cudaStream_t s) {
     state_layout<T>(p, &sc);
     long long longest = 1;
     for (int k = 0; k < sc.n; ++k) longest = std::max(longest, sc.len[k]);
-    const dim3 grid((unsigned)std::min<long long>((longest + 255) / 256, 1184), (unsigned)std::max(1, sc.n));
+    const dim3 grid((unsigned)std::min<long long>((longest * (long long)sizeof(T) / 16 + 255) / 256 + 1, 1184), (unsigned)std::max(1, sc.n));
     k_state_copy<T><<<grid, 256, 0, s>>>(sc, slot, p->grid<T>().counter, save ? 1 : 0);
     TFD_CUDA(cudaGetLastError());
     return TFD_OK;
@@ -2622,6 +2627,7 @@ int adjoint_create_t(tfd_adjoint *adj, cudaStream_t s) {
         for (int j = 0; j < 2; ++j) A.sPsiE[a][j] = m.sPsiE[a][j];
     if (int rc = slab_bounds(p, A.slab)) return rc;
     A.split = pass_split<T>(p, -1, 1);
+    if (!p->two_pass) TFD_CHECK(setup_pass<T>(p));       // replays run as two passes whatever the plan's kernel
     if (A.g.n[2] > 65535) return fail(TFD_ERR_UNSUPPORTED, "the adjoint step launches one z plane per grid row: nz above 65535");
     adj->used = adjoint_layout<T>(p, &A, adj->arena);
     TFD_CUDA(cudaMemsetAsync(adj->arena, 0, adj->used, s));
@@ -2655,6 +2661,35 @@ int adjoint_step_t(tfd_adjoint *adj, const void *snapshot, const void *seeds, cu
     }
     TFD_CUDA(cudaGetLastError());
     adj->q ^= 1;
+    return TFD_OK;
+}
+
+// Restores the checkpoint of a segment of `count` steps, replays all but the last step (each leaving its H and E-family
+// CPML memories in its slot of `replay`) and transposes the steps in reverse. The checkpoint is the first step's snapshot.
+template <typename T>
+int adjoint_segment_t(tfd_adjoint *adj, const char *checkpoint, int count, char *replay, size_t slot_bytes, const T *seeds, cudaStream_t s) {
+    tfd_plan *p = adj->p;
+    const AdjArgs<T> &A = adj->args<T>();
+    TFD_CHECK(state_copy_t<T>(p, const_cast<char *>(checkpoint), false, s));
+    PassArgs<T> a = p->pass<T>();
+    a.g.counter = p->grid<T>().counter;
+    a.snap.stride = (long long)(slot_bytes / sizeof(T));
+    for (int c = 0; c < 3; ++c) a.snap.sH[c] = A.sH[c];
+    for (int ax = 0; ax < 3; ++ax)
+        for (int j = 0; j < 2; ++j) a.snap.sPsiE[ax][j] = A.sPsiE[ax][j];
+    if (p->pass_ctas > 0 && count > 1) {
+        a.snap.base = (T *)(replay + slot_bytes);
+        TFD_CHECK(launch_pass_steps<T>(p, a, count - 1, false, s));
+    } else {
+        for (int j = 1; j < count; ++j) {
+            a.snap.base = (T *)(replay + j * slot_bytes);
+            TFD_CHECK(launch_two_pass<T>(p, a, s));
+            k_pass_advance<T><<<1, 1, 0, s>>>(a.g);
+        }
+    }
+    for (int j = count - 1; j >= 0; --j)
+        TFD_CHECK(adjoint_step_t<T>(adj, j == 0 ? checkpoint : replay + j * slot_bytes, seeds ? seeds + (size_t)j * p->desc.n_traces : nullptr, s));
+    TFD_CUDA(cudaGetLastError());
     return TFD_OK;
 }
 
@@ -2745,6 +2780,20 @@ int tfd_adjoint_step(tfd_adjoint *adj, const void *snapshot, const void *seeds, 
     if (!adj || !snapshot || ((uintptr_t)snapshot & 255)) return fail(TFD_ERR_INVALID, "bad adjoint step arguments");
     return adj->p->desc.precision == 8 ? adjoint_step_t<double>(adj, snapshot, seeds, as_stream(stream))
                                        : adjoint_step_t<float>(adj, snapshot, seeds, as_stream(stream));
+}
+
+int tfd_adjoint_segment(tfd_adjoint *adj, const void *checkpoint, int32_t count, void *replay, size_t slot_bytes, const void *seeds,
+                        void *stream) {
+    if (!adj || !checkpoint || ((uintptr_t)checkpoint & 255) || count < 1 || (count > 1 && (!replay || ((uintptr_t)replay & 255))) ||
+        (slot_bytes & 255))
+        return fail(TFD_ERR_INVALID, "bad adjoint segment arguments");
+    size_t need = 0;
+    tfd_state_bytes(adj->p, &need);
+    if (slot_bytes < need) return fail(TFD_ERR_INVALID, "replay slots shorter than tfd_state_bytes()");
+    if (adj->p->in_batch) return fail(TFD_ERR_INVALID, "this plan belongs to a batch");
+    return adj->p->desc.precision == 8
+               ? adjoint_segment_t<double>(adj, (const char *)checkpoint, count, (char *)replay, slot_bytes, (const double *)seeds, as_stream(stream))
+               : adjoint_segment_t<float>(adj, (const char *)checkpoint, count, (char *)replay, slot_bytes, (const float *)seeds, as_stream(stream));
 }
 
 int tfd_adjoint_sensitivity(tfd_adjoint *adj, void *dst, int where, void *stream) {

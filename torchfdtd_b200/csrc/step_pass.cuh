@@ -42,12 +42,22 @@ template <typename T> constexpr int kPassBlocks = sizeof(T) == 4 ? 3 : 2;
 // 290 us per step).
 struct PassSplit { int plain, x_lo, slab; unsigned magic_plain, magic_slab, plain_total, total; };
 
+// Where the steps of a replay leave what their transposes read: H and the E-family CPML memories after each step, in the
+// restart-snapshot layout (element offsets from the slot's start). base: the slot after the launch's first step.
+template <typename T>
+struct PassSnap {
+    T *base;                     // nullptr: no replay
+    long long stride;            // elements between slots
+    long long sH[3], sPsiE[3][2];
+};
+
 template <typename T>
 struct PassArgs {
     Grid<T> g;
     int slab[2][3][4];           // per family and axis: lo0, hi0, lo1, hi1 of the two CPML slabs
     int tables;                  // 1: more than two slabs on some axis, slab rows come from the row tables
     PassSplit split[2];          // per family
+    PassSnap<T> snap;
 };
 
 template <typename T> struct alignas(16) Pack { static constexpr int N = 16 / sizeof(T); T v[N]; };
@@ -111,21 +121,22 @@ __device__ __forceinline__ void slab_load(const PassArgs<T> &A, const PassCell<I
     }
 }
 
-// psi <- b psi + c d (stored to out); d <- d/kappa + psi, for term j of the x axis.
+// psi <- b psi + c d (stored to out, and to the replay's slot); d <- d/kappa + psi, for term j of the x axis.
 template <typename T, typename I>
-__device__ __forceinline__ void slab_apply(const PassSlab<T, I> &m, int j, T *out, T (&d)[Pack<T>::N]) {
+__device__ __forceinline__ void slab_apply(const PassSlab<T, I> &m, int j, T *out, T *snap, T (&d)[Pack<T>::N]) {
 #pragma unroll
     for (int k = 0; k < Pack<T>::N; ++k)
         if (m.row[k] >= 0) {
             const T v = m.old[j][k] * m.b[k] + m.c[k] * d[k];
             out[m.at + m.row[k]] = v;
+            if (snap != nullptr) snap[m.at + m.row[k]] = v;
             d[k] = d[k] * m.k[k] + v;
         }
 }
 
 // The same for a y or z slab row r >= 0 (axis a) of a group: one memory vector per term.
 template <typename T, int F, int a, typename I>
-__device__ __forceinline__ void pass_cpml(const PassArgs<T> &A, const PassCell<I> &q, int r, const T *old, T *out, T (&d)[Pack<T>::N]) {
+__device__ __forceinline__ void pass_cpml(const PassArgs<T> &A, const PassCell<I> &q, int r, const T *old, T *out, T *snap, T (&d)[Pack<T>::N]) {
     const Grid<T> &g = A.g;
     const int c = a == 1 ? q.y : q.z;
     const I p = a == 1 ? ((I)q.z * g.rows[F][1] + r) * g.pitch + q.x : ((I)r * g.n[1] + q.y) * g.pitch + q.x;
@@ -137,6 +148,7 @@ __device__ __forceinline__ void pass_cpml(const PassArgs<T> &A, const PassCell<I
         d[k] = d[k] * ck + m.v[k];
     }
     pack_store(out + p, m);
+    if (snap != nullptr) pack_store(snap + p, m);
 }
 
 // Dispersive samples (threads j of total): the coupled trapezoidal ADE turns the free update that the E pass stored into
@@ -213,7 +225,7 @@ __device__ __forceinline__ void pass_sources(const Grid<T> &g, int family, long 
 
 // E_new of a group. ACTIVE: bitmask of advanced components (bit c: E_c, bit 3+c: H_c). XS: the group meets an x slab.
 template <typename T, int ACTIVE, bool METRIC, bool ADE, bool XS, typename I>
-__device__ __forceinline__ void pass_e(const PassArgs<T> &A, const PassCell<I> &q, int par, long long n) {
+__device__ __forceinline__ void pass_e(const PassArgs<T> &A, const PassCell<I> &q, int par, long long n, T *slot) {
     constexpr int N = Pack<T>::N;
     const Grid<T> &g = A.g;
     constexpr bool HX = ACTIVE & 8, HY = ACTIVE & 16, HZ = ACTIVE & 32;
@@ -266,7 +278,7 @@ __device__ __forceinline__ void pass_e(const PassArgs<T> &A, const PassCell<I> &
             if (k == 0 && !xin) d[k] = T(0);
             if (METRIC) d[k] = d[k] * mx[k];
         }
-        if (XS) slab_apply(sx, j, g.psiE[par ^ 1][0][j], d);
+        if (XS) slab_apply(sx, j, g.psiE[par ^ 1][0][j], slot ? slot + A.snap.sPsiE[0][j] : nullptr, d);
     };
     auto dy = [&](const Pack<T> &h, const Pack<T> &low, int j, T (&d)[N]) {
 #pragma unroll
@@ -278,7 +290,7 @@ __device__ __forceinline__ void pass_e(const PassArgs<T> &A, const PassCell<I> &
             if (!yin)
 #pragma unroll
                 for (int k = 0; k < N; ++k) d[k] = T(0);
-            if (ry >= 0) pass_cpml<T, 0, 1>(A, q, ry, g.psiE[par][1][j], g.psiE[par ^ 1][1][j], d);
+            if (ry >= 0) pass_cpml<T, 0, 1>(A, q, ry, g.psiE[par][1][j], g.psiE[par ^ 1][1][j], slot ? slot + A.snap.sPsiE[1][j] : nullptr, d);
         }
     };
     auto dz = [&](const Pack<T> &h, const Pack<T> &low, int j, T (&d)[N]) {
@@ -291,7 +303,7 @@ __device__ __forceinline__ void pass_e(const PassArgs<T> &A, const PassCell<I> &
             if (!zin)
 #pragma unroll
                 for (int k = 0; k < N; ++k) d[k] = T(0);
-            if (rz >= 0) pass_cpml<T, 0, 2>(A, q, rz, g.psiE[par][2][j], g.psiE[par ^ 1][2][j], d);
+            if (rz >= 0) pass_cpml<T, 0, 2>(A, q, rz, g.psiE[par][2][j], g.psiE[par ^ 1][2][j], slot ? slot + A.snap.sPsiE[2][j] : nullptr, d);
         }
     };
     T d0[N], d1[N];
@@ -334,7 +346,7 @@ __device__ __forceinline__ void pass_e(const PassArgs<T> &A, const PassCell<I> &
 
 // H_new of a group from the stored E_new.
 template <typename T, int ACTIVE, bool METRIC, bool XS, typename I>
-__device__ __forceinline__ void pass_h(const PassArgs<T> &A, const PassCell<I> &q, int par, long long n) {
+__device__ __forceinline__ void pass_h(const PassArgs<T> &A, const PassCell<I> &q, int par, long long n, T *slot) {
     constexpr int N = Pack<T>::N;
     const Grid<T> &g = A.g;
     constexpr bool HX = ACTIVE & 8, HY = ACTIVE & 16, HZ = ACTIVE & 32;
@@ -388,7 +400,7 @@ __device__ __forceinline__ void pass_h(const PassArgs<T> &A, const PassCell<I> &
                     d[k] = g.periodic[0] ? right - f.v[k] : (g.pec_on[0] ? g.pec_neg[0] * f.v[k] : T(0));
                     if (METRIC && g.periodic[0]) d[k] = d[k] * mx[k];
                 }
-        if (XS) slab_apply(sx, j, g.psiH[0][j], d);
+        if (XS) slab_apply(sx, j, g.psiH[0][j], (T *)nullptr, d);
     };
     auto edge = [&](int a, const Pack<T> &f, T (&d)[N]) {       // no +1 neighbour and no period: the PEC ghost, or 0
 #pragma unroll
@@ -402,7 +414,7 @@ __device__ __forceinline__ void pass_h(const PassArgs<T> &A, const PassCell<I> &
         }
         if (ycold) {
             if (!yin && !g.periodic[1]) edge(1, f, d);
-            if (ry >= 0) pass_cpml<T, 1, 1>(A, q, ry, g.psiH[1][j], g.psiH[1][j], d);
+            if (ry >= 0) pass_cpml<T, 1, 1>(A, q, ry, g.psiH[1][j], g.psiH[1][j], (T *)nullptr, d);
         }
     };
     auto dz = [&](const Pack<T> &f, const Pack<T> &high, int j, T (&d)[N]) {
@@ -413,7 +425,7 @@ __device__ __forceinline__ void pass_h(const PassArgs<T> &A, const PassCell<I> &
         }
         if (zcold) {
             if (!zin && !g.periodic[2]) edge(2, f, d);
-            if (rz >= 0) pass_cpml<T, 1, 2>(A, q, rz, g.psiH[2][j], g.psiH[2][j], d);
+            if (rz >= 0) pass_cpml<T, 1, 2>(A, q, rz, g.psiH[2][j], g.psiH[2][j], (T *)nullptr, d);
         }
     };
     T d0[N], d1[N];
@@ -450,6 +462,7 @@ __device__ __forceinline__ void pass_h(const PassArgs<T> &A, const PassCell<I> &
             for (int k = 0; k < N; ++k)
                 if (q.x + k >= nx) h[c].v[k] = T(0);
         pack_store(g.H[par ^ 1][c] + i, h[c]);
+        if (slot != nullptr) pack_store(slot + A.snap.sH[c] + i, h[c]);
     }
 }
 
@@ -488,21 +501,21 @@ __device__ __forceinline__ PassCell<I> pass_cell(const Grid<T> &g, const PassSpl
 
 // Group p of plane z in each pass.
 template <typename T, int ACTIVE, bool METRIC, bool ADE, typename I>
-__device__ __forceinline__ void pass_block_e(const PassArgs<T> &A, unsigned p, int z, int par, long long n) {
+__device__ __forceinline__ void pass_block_e(const PassArgs<T> &A, unsigned p, int z, int par, long long n, T *slot) {
     if (p >= A.split[0].total) return;
     const bool slab = p >= A.split[0].plain_total;
     const PassCell<I> q = pass_cell<I>(A.g, A.split[0], p, z, slab);
-    if (slab) pass_e<T, ACTIVE, METRIC, ADE, true>(A, q, par, n);
-    else pass_e<T, ACTIVE, METRIC, ADE, false>(A, q, par, n);
+    if (slab) pass_e<T, ACTIVE, METRIC, ADE, true>(A, q, par, n, slot);
+    else pass_e<T, ACTIVE, METRIC, ADE, false>(A, q, par, n, slot);
 }
 
 template <typename T, int ACTIVE, bool METRIC, typename I>
-__device__ __forceinline__ void pass_block_h(const PassArgs<T> &A, unsigned p, int z, int par, long long n) {
+__device__ __forceinline__ void pass_block_h(const PassArgs<T> &A, unsigned p, int z, int par, long long n, T *slot) {
     if (p >= A.split[1].total) return;
     const bool slab = p >= A.split[1].plain_total;
     const PassCell<I> q = pass_cell<I>(A.g, A.split[1], p, z, slab);
-    if (slab) pass_h<T, ACTIVE, METRIC, true>(A, q, par, n);
-    else pass_h<T, ACTIVE, METRIC, false>(A, q, par, n);
+    if (slab) pass_h<T, ACTIVE, METRIC, true>(A, q, par, n, slot);
+    else pass_h<T, ACTIVE, METRIC, false>(A, q, par, n, slot);
 }
 
 // One launch per pass: blocks of kPassThreads groups of one plane (blockIdx.x), planes on
@@ -512,7 +525,7 @@ __global__ void __launch_bounds__(kPassThreads, kPassBlocks<T>) k_pass_e(const _
     const long long n = *A.g.counter;
     if (n >= A.g.steps) return;                 // past the plan's last step: a step is a no-op
     for (int z = blockIdx.y; z < A.g.n[2]; z += gridDim.y)
-        pass_block_e<T, ACTIVE, METRIC, ADE, I>(A, blockIdx.x * kPassThreads + threadIdx.x, z, (int)(n & 1), n);
+        pass_block_e<T, ACTIVE, METRIC, ADE, I>(A, blockIdx.x * kPassThreads + threadIdx.x, z, (int)(n & 1), n, A.snap.base);
 }
 
 template <typename T, int ACTIVE, bool METRIC, typename I>
@@ -520,7 +533,14 @@ __global__ void __launch_bounds__(kPassThreads, kPassBlocks<T>) k_pass_h(const _
     const long long n = *A.g.counter;
     if (n >= A.g.steps) return;
     for (int z = A.g.n[2] - 1 - (int)blockIdx.y; z >= 0; z -= gridDim.y)
-        pass_block_h<T, ACTIVE, METRIC, I>(A, blockIdx.x * kPassThreads + threadIdx.x, z, (int)(n & 1), n);
+        pass_block_h<T, ACTIVE, METRIC, I>(A, blockIdx.x * kPassThreads + threadIdx.x, z, (int)(n & 1), n, A.snap.base);
+}
+
+// The step counter alone (a replayed step records no observations).
+template <typename T>
+__global__ void k_pass_advance(const __grid_constant__ Grid<T> g) {
+    const long long n = *g.counter;
+    if (n < g.steps) *g.counter = n + 1;
 }
 
 // ---- many steps in one launch ----------------------------------------------------------------------------------
@@ -574,17 +594,18 @@ __global__ void __launch_bounds__(kPassStepThreads, 1) k_pass_steps(const __grid
     long long n = n0;
     for (int k = 0; k < count && n < g.steps; ++k, ++n) {
         const int par = (int)(n & 1);
+        T *slot = A.snap.base != nullptr ? A.snap.base + k * A.snap.stride : nullptr;
         if (k > 0)
             for (int b = blockIdx.x; b < mgx * mgy; b += gridDim.x) monitor_work(m, b % mgx, b / mgx, n - 1, mgx);
         for (int it = blockIdx.x; it < items; it += gridDim.x)
-            pass_block_e<T, ACTIVE, METRIC, ADE, int>(A, (it % per_plane) * kPassStepThreads + threadIdx.x, it / per_plane, par, n);
+            pass_block_e<T, ACTIVE, METRIC, ADE, int>(A, (it % per_plane) * kPassStepThreads + threadIdx.x, it / per_plane, par, n, slot);
         if (!barrier()) return;
         if (ADE) {
             for (int j = blockIdx.x * kPassStepThreads + threadIdx.x; j < g.ade_samples; j += gridDim.x * kPassStepThreads) pass_ade(g, j, par, n);
             if (!barrier()) return;
         }
         for (int it = blockIdx.x; it < items; it += gridDim.x)
-            pass_block_h<T, ACTIVE, METRIC, int>(A, (it % per_plane) * kPassStepThreads + threadIdx.x, it / per_plane, par, n);
+            pass_block_h<T, ACTIVE, METRIC, int>(A, (it % per_plane) * kPassStepThreads + threadIdx.x, it / per_plane, par, n, slot);
         if (!barrier()) return;
     }
     if (n > n0)

@@ -110,6 +110,7 @@ SIGNATURES = {
     'tfd_adjoint_create': (ctypes.c_int, [c_vp, c_vp, ctypes.c_size_t, c_vp, ctypes.POINTER(c_vp)]),
     'tfd_adjoint_reset': (ctypes.c_int, [c_vp, c_vp]),
     'tfd_adjoint_step': (ctypes.c_int, [c_vp, c_vp, c_vp, c_vp]),
+    'tfd_adjoint_segment': (ctypes.c_int, [c_vp, c_vp, c_i32, c_vp, ctypes.c_size_t, c_vp, c_vp]),
     'tfd_adjoint_sensitivity': (ctypes.c_int, [c_vp, c_vp, ctypes.c_int, c_vp]),
     'tfd_adjoint_destroy': (None, [c_vp]),
     'tfd_error_string': (ctypes.c_char_p, [ctypes.c_int]),
@@ -660,6 +661,12 @@ class NativeAdjoint:
         """Transpose the step that left ``snapshot``'s state, after adding ``seeds`` (one per trace)."""
         check(library().tfd_adjoint_step(self.handle, c_vp(snapshot.data_ptr()),
                                          c_vp(seeds.data_ptr()) if seeds is not None else None, _stream(stream)))
+
+    def segment(self, checkpoint, count, replay, seeds=None, stream=None):
+        """Replay the ``count`` steps after ``checkpoint`` into the rows of ``replay`` and transpose them in reverse;
+        ``seeds``: (count, traces) contiguous device tensor, or None."""
+        check(library().tfd_adjoint_segment(self.handle, c_vp(checkpoint.data_ptr()), int(count), c_vp(replay.data_ptr()),
+                                            replay.shape[1], c_vp(seeds.data_ptr()) if seeds is not None else None, _stream(stream)))
 
     def sensitivity(self):
         """S = sum over steps of e_bar * curl_b(H), (nx, ny, nz, 3) torch tensor on the device."""
