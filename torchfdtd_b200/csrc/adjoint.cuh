@@ -73,13 +73,13 @@ __device__ __forceinline__ Pack<double> pack_ldg(const double *p) {
 
 // CPML transpose of the D values v[] of a group's cells in one y or z slab row r: m = psi_bar + v; psi_bar <- b m (when
 // own); v <- v / kappa + c m.
-template <typename T, int F, int a>
+template <typename I, int F, int a, typename T>
 __device__ __forceinline__ void adj_slab_row_apply(const AdjArgs<T> &A, int r, int x, int y, int z, const T *old, T *out, bool own,
                                                    T (&v)[Pack<T>::N]) {
     constexpr int N = Pack<T>::N;
     const Grid<T> &g = A.g;
     const int c = a == 1 ? y : z;
-    const long long p = g.psi_index(a, x, y, z, r, g.rows[F][a]);
+    const I p = a == 1 ? ((I)z * g.rows[F][1] + r) * g.pitch + x : ((I)r * g.n[1] + y) * g.pitch + x;
     const T b = __ldg(g.cb[F][a] + c), cc = __ldg(g.cc[F][a] + c), ck = __ldg(g.ck[F][a] + c);
     const Pack<T> m0 = pack_ldg(old + p);
     Pack<T> w;
@@ -93,31 +93,32 @@ __device__ __forceinline__ void adj_slab_row_apply(const AdjArgs<T> &A, int r, i
 }
 
 // The same for one cell of an x slab.
-template <typename T, int F>
+template <typename I, int F, typename T>
 __device__ __forceinline__ T adj_slab_x_apply(const AdjArgs<T> &A, int x, int y, int z, const T *old, T *out, bool own, T v) {
     const Grid<T> &g = A.g;
     if (old == nullptr || x < 0 || x >= g.n[0]) return v;
     const int r = adj_slab_row(A.slab[F][0], x);
     if (r < 0) return v;
-    const long long p = g.psi_index(0, x, y, z, r, g.rows[F][0]);
+    const I p = ((I)z * g.n[1] + y) * g.rows[F][0] + r;
     const T m = __ldg(old + p) + v;
     if (own) out[p] = __ldg(g.cb[F][0] + x) * m;
     return v * __ldg(g.ck[F][0] + x) + __ldg(g.cc[F][0] + x) * m;
 }
 
-// e_bar_new and the sensitivity of a group. XS: the group or a neighbour of its ends lies in an x slab.
+// e_bar_new and the sensitivity of a group. XS: the group or a neighbour of its ends lies in an x slab. YZ: its row may meet
+// a y or z slab or face, or the mesh is nonuniform; false (the plain variant) leaves those cases' code out.
 // The D values of H-family terms are sign * (-cn h_bar): through the CPML transpose below the last cell, one period away
 // or the PEC edge at it; e_bar[c] += D(c - 1), e_bar[c] -= D(c), in the order of the terms.
-template <typename T, int ACTIVE, bool XS>
-__device__ __forceinline__ void adj_pass_e(const AdjArgs<T> &A, const T *__restrict__ slot, int q, const PassCell<long long> &w) {
+template <typename T, int ACTIVE, bool XS, bool YZ, typename I>
+__device__ __forceinline__ void adj_pass_e(const AdjArgs<T> &A, const T *__restrict__ slot, int q, const PassCell<I> &w) {
     constexpr int N = Pack<T>::N;
     const Grid<T> &g = A.g;
-    const long long i = w.i;
+    const I i = w.i, plane = (I)g.plane;
     const int x = w.x, y = w.y, z = w.z, nx = g.n[0], ny = g.n[1], nz = g.n[2];
     const bool last = x + N >= nx;
-    const long long ix = x > 0 ? i - 1 : i + (g.periodic[0] ? nx - 1 : 0);
-    const long long iy = y > 0 ? i - g.pitch : i + (g.periodic[1] ? (long long)(ny - 1) * g.pitch : 0);
-    const long long iz = z > 0 ? i - g.plane : i + (g.periodic[2] ? (long long)(nz - 1) * g.plane : 0);
+    const I ix = x > 0 ? i - 1 : i + (g.periodic[0] ? nx - 1 : 0);
+    const I iy = !YZ || y > 0 ? i - g.pitch : i + (g.periodic[1] ? (I)(ny - 1) * g.pitch : 0);
+    const I iz = !YZ || z > 0 ? i - plane : i + (g.periodic[2] ? (I)(nz - 1) * plane : 0);
     Pack<T> h[3], hy[3], hz[3], f[3], fy[3], fz[3], eb[3], S[3];
     T hx[3], fx[3];
 #pragma unroll
@@ -137,7 +138,7 @@ __device__ __forceinline__ void adj_pass_e(const AdjArgs<T> &A, const T *__restr
             S[c] = pack_load(A.S[c] + i);
         }
     }
-    const bool metric = g.metric[0][0] != nullptr || g.metric[0][1] != nullptr || g.metric[0][2] != nullptr;
+    const bool metric = YZ && (g.metric[0][0] != nullptr || g.metric[0][1] != nullptr || g.metric[0][2] != nullptr);
     auto mt = [&](int fam, int a, int c) -> T { return g.metric[fam][a] != nullptr ? g.metric[fam][a][c] : T(1); };
     Pack<T> e[3];
 #pragma unroll
@@ -162,13 +163,29 @@ __device__ __forceinline__ void adj_pass_e(const AdjArgs<T> &A, const T *__restr
             }
             const T *old = A.pHb[q][a][t.j];
             T *out = A.pHb[q ^ 1][a][t.j];
-            if (a == 0) {
+            // Away from the faces of the axis (the usual case): both values, nothing else.
+            if (a == 0 && x > 0 && !last) {
 #pragma unroll
                 for (int k = 0; k < N; ++k) {
                     const int c = x + k;
                     if (XS) {
-                        if (c >= 1) lo[k] = adj_slab_x_apply<T, 1>(A, c - 1, y, z, old, out, false, lo[k]);
-                        if (c < nx - 1) up[k] = adj_slab_x_apply<T, 1>(A, c, y, z, old, out, true, up[k]);
+                        lo[k] = adj_slab_x_apply<I, 1>(A, c - 1, y, z, old, out, false, lo[k]);
+                        up[k] = adj_slab_x_apply<I, 1>(A, c, y, z, old, out, true, up[k]);
+                    }
+                    if (metric) {
+                        lo[k] = lo[k] * mt(1, 0, c - 1);
+                        up[k] = up[k] * mt(1, 0, c);
+                    }
+                    contrib[k] = contrib[k] + lo[k];
+                    contrib[k] = contrib[k] - up[k];
+                }
+            } else if (a == 0) {
+#pragma unroll
+                for (int k = 0; k < N; ++k) {
+                    const int c = x + k;
+                    if (XS) {
+                        if (c >= 1) lo[k] = adj_slab_x_apply<I, 1>(A, c - 1, y, z, old, out, false, lo[k]);
+                        if (c < nx - 1) up[k] = adj_slab_x_apply<I, 1>(A, c, y, z, old, out, true, up[k]);
                     }
                     if (metric && c < nx) {
                         lo[k] = lo[k] * mt(1, 0, c >= 1 ? c - 1 : nx - 1);
@@ -189,21 +206,41 @@ __device__ __forceinline__ void adj_pass_e(const AdjArgs<T> &A, const T *__restr
                 }
             } else {
                 const int c = a == 1 ? y : z, n = g.n[a];
+                if (!YZ) {
+#pragma unroll
+                    for (int k = 0; k < N; ++k) {
+                        contrib[k] = contrib[k] + lo[k];
+                        contrib[k] = contrib[k] - up[k];
+                    }
+                    continue;
+                }
                 if (c >= 1 && old != nullptr) {
                     const int r = adj_slab_row(A.slab[1][a], c - 1);
                     if (r >= 0) {
-                        if (a == 1) adj_slab_row_apply<T, 1, 1>(A, r, x, y - 1, z, old, out, false, lo);
-                        else adj_slab_row_apply<T, 1, 2>(A, r, x, y, z - 1, old, out, false, lo);
+                        if (a == 1) adj_slab_row_apply<I, 1, 1>(A, r, x, y - 1, z, old, out, false, lo);
+                        else adj_slab_row_apply<I, 1, 2>(A, r, x, y, z - 1, old, out, false, lo);
                     }
                 }
                 if (c < n - 1 && old != nullptr) {
                     const int r = adj_slab_row(A.slab[1][a], c);
                     if (r >= 0) {
-                        if (a == 1) adj_slab_row_apply<T, 1, 1>(A, r, x, y, z, old, out, true, up);
-                        else adj_slab_row_apply<T, 1, 2>(A, r, x, y, z, old, out, true, up);
+                        if (a == 1) adj_slab_row_apply<I, 1, 1>(A, r, x, y, z, old, out, true, up);
+                        else adj_slab_row_apply<I, 1, 2>(A, r, x, y, z, old, out, true, up);
                     }
                 }
                 const T ml = metric ? mt(1, a, c >= 1 ? c - 1 : n - 1) : T(1), mu = metric ? mt(1, a, c) : T(1);
+                if (c >= 1 && c < n - 1) {
+#pragma unroll
+                    for (int k = 0; k < N; ++k) {
+                        if (metric) {
+                            lo[k] = lo[k] * ml;
+                            up[k] = up[k] * mu;
+                        }
+                        contrib[k] = contrib[k] + lo[k];
+                        contrib[k] = contrib[k] - up[k];
+                    }
+                    continue;
+                }
                 const bool pec = c == n - 1 && !g.periodic[a] && g.pec_on[a], none = c == n - 1 && !g.periodic[a] && !g.pec_on[a];
 #pragma unroll
                 for (int k = 0; k < N; ++k) {
@@ -228,7 +265,7 @@ __device__ __forceinline__ void adj_pass_e(const AdjArgs<T> &A, const T *__restr
             if (g.n[a] == 1) continue;
             T d[N];
             const int c0 = a == 0 ? x : a == 1 ? y : z;
-            const bool live = c0 > 0 || g.periodic[a];
+            const bool live = (a != 0 && !YZ) || c0 > 0 || g.periodic[a];
 #pragma unroll
             for (int k = 0; k < N; ++k) {
                 const T below = a == 0 ? (k == 0 ? fx[in] : f[in].v[k == 0 ? 0 : k - 1]) : a == 1 ? fy[in].v[k] : fz[in].v[k];
@@ -236,7 +273,7 @@ __device__ __forceinline__ void adj_pass_e(const AdjArgs<T> &A, const T *__restr
                 if ((a != 0 || k == 0) && !live) d[k] = T(0);
                 if (metric) d[k] = d[k] * mt(0, a, a == 0 ? min(x + k, nx - 1) : c0);
             }
-            if (A.sPsiE[a][t.j] >= 0) {
+            if ((a == 0 ? XS : YZ) && A.sPsiE[a][t.j] >= 0) {
                 const T *psi = slot + A.sPsiE[a][t.j];
                 if (a == 0) {
                     if (XS)
@@ -244,14 +281,14 @@ __device__ __forceinline__ void adj_pass_e(const AdjArgs<T> &A, const T *__restr
                         for (int k = 0; k < N; ++k) {
                             const int c = x + k, r = c < nx ? adj_slab_row(A.slab[0][0], c) : -1;
                             if (c > 0 && r >= 0) {
-                                const T m = __ldg(psi + g.psi_index(0, c, y, z, r, g.rows[0][0])) * __ldg(g.cb[0][0] + c) + __ldg(g.cc[0][0] + c) * d[k];
+                                const T m = __ldg(psi + (((I)z * ny + y) * g.rows[0][0] + r)) * __ldg(g.cb[0][0] + c) + __ldg(g.cc[0][0] + c) * d[k];
                                 d[k] = d[k] * __ldg(g.ck[0][0] + c) + m;
                             }
                         }
                 } else {
                     const int r = c0 > 0 ? adj_slab_row(A.slab[0][a], c0) : -1;
                     if (r >= 0) {
-                        const Pack<T> m0 = pack_ldg(psi + g.psi_index(a, x, y, z, r, g.rows[0][a]));
+                        const Pack<T> m0 = pack_ldg(psi + (a == 1 ? ((I)z * g.rows[0][1] + r) * g.pitch + x : ((I)r * ny + y) * g.pitch + x));
                         const T b = __ldg(g.cb[0][a] + c0), cc = __ldg(g.cc[0][a] + c0), ck = __ldg(g.ck[0][a] + c0);
 #pragma unroll
                         for (int k = 0; k < N; ++k) {
@@ -267,7 +304,7 @@ __device__ __forceinline__ void adj_pass_e(const AdjArgs<T> &A, const T *__restr
 #pragma unroll
         for (int k = 0; k < N; ++k) {
             S[C].v[k] = S[C].v[k] + e[C].v[k] * acc[k];
-            if (x + k >= nx) e[C].v[k] = S[C].v[k] = T(0);
+            if (last && x + k >= nx) e[C].v[k] = S[C].v[k] = T(0);
         }
     }
 #pragma unroll
@@ -280,16 +317,16 @@ __device__ __forceinline__ void adj_pass_e(const AdjArgs<T> &A, const T *__restr
 
 // h_bar_new of a group from the stored e_bar_new. The D values of E-family terms are sign * ((cn / eps) e_bar_new), zero
 // at cell 0 without a period; h_bar[c] += D(c), h_bar[c] -= D(c + 1).
-template <typename T, int ACTIVE, bool XS>
-__device__ __forceinline__ void adj_pass_h(const AdjArgs<T> &A, int q, const PassCell<long long> &w) {
+template <typename T, int ACTIVE, bool XS, bool YZ, typename I>
+__device__ __forceinline__ void adj_pass_h(const AdjArgs<T> &A, int q, const PassCell<I> &w) {
     constexpr int N = Pack<T>::N;
     const Grid<T> &g = A.g;
-    const long long i = w.i;
+    const I i = w.i, plane = (I)g.plane;
     const int x = w.x, y = w.y, z = w.z, nx = g.n[0], ny = g.n[1], nz = g.n[2];
     const bool last = x + N >= nx;
-    const long long ix = last ? i - x : i + N;
-    const long long iy = y < ny - 1 ? i + g.pitch : i - (g.periodic[1] ? (long long)(ny - 1) * g.pitch : 0);
-    const long long iz = z < nz - 1 ? i + g.plane : i - (g.periodic[2] ? (long long)(nz - 1) * g.plane : 0);
+    const I ix = last ? i - x : i + N;
+    const I iy = !YZ || y < ny - 1 ? i + g.pitch : i - (g.periodic[1] ? (I)(ny - 1) * g.pitch : 0);
+    const I iz = !YZ || z < nz - 1 ? i + plane : i - (g.periodic[2] ? (I)(nz - 1) * plane : 0);
     // u = (cn / eps) e_bar_new at the cells and at the +x, +y, +z neighbours.
     Pack<T> u[3], uy[3], uz[3], hb[3];
     T ux[3];
@@ -312,7 +349,7 @@ __device__ __forceinline__ void adj_pass_h(const AdjArgs<T> &A, int q, const Pas
         }
         if ((ACTIVE >> (3 + c)) & 1) hb[c] = pack_ldg(A.hb[q][c] + i);
     }
-    const bool metric = g.metric[0][0] != nullptr || g.metric[0][1] != nullptr || g.metric[0][2] != nullptr;
+    const bool metric = YZ && (g.metric[0][0] != nullptr || g.metric[0][1] != nullptr || g.metric[0][2] != nullptr);
     auto mt = [&](int a, int c) -> T { return g.metric[0][a] != nullptr ? g.metric[0][a][c] : T(1); };
 #pragma unroll
     for (int C = 0; C < 3; ++C) {
@@ -334,7 +371,22 @@ __device__ __forceinline__ void adj_pass_h(const AdjArgs<T> &A, int q, const Pas
             }
             const T *old = A.pEb[q][a][t.j];
             T *out = A.pEb[q ^ 1][a][t.j];
-            if (a == 0) {
+            if (a == 0 && x > 0 && !last) {
+#pragma unroll
+                for (int k = 0; k < N; ++k) {
+                    const int c = x + k;
+                    if (XS) {
+                        at[k] = adj_slab_x_apply<I, 0>(A, c, y, z, old, out, true, at[k]);
+                        up[k] = adj_slab_x_apply<I, 0>(A, c + 1, y, z, old, out, false, up[k]);
+                    }
+                    if (metric) {
+                        at[k] = at[k] * mt(0, c);
+                        up[k] = up[k] * mt(0, c + 1);
+                    }
+                    contrib[k] = contrib[k] + at[k];
+                    contrib[k] = contrib[k] - up[k];
+                }
+            } else if (a == 0) {
                 if (last && g.periodic[0]) {             // the last cell's +1 neighbour is the row's first
                     const T first = t.sign > 0 ? ux[o] : -ux[o];
 #pragma unroll
@@ -345,8 +397,8 @@ __device__ __forceinline__ void adj_pass_h(const AdjArgs<T> &A, int q, const Pas
                 for (int k = 0; k < N; ++k) {
                     const int c = x + k;
                     if (XS) {
-                        if (c >= 1) at[k] = adj_slab_x_apply<T, 0>(A, c, y, z, old, out, true, at[k]);
-                        if (c + 1 <= nx - 1) up[k] = adj_slab_x_apply<T, 0>(A, c + 1, y, z, old, out, false, up[k]);
+                        if (c >= 1) at[k] = adj_slab_x_apply<I, 0>(A, c, y, z, old, out, true, at[k]);
+                        if (c + 1 <= nx - 1) up[k] = adj_slab_x_apply<I, 0>(A, c + 1, y, z, old, out, false, up[k]);
                     }
                     if (metric && c < nx) {
                         at[k] = at[k] * mt(0, c);
@@ -360,21 +412,41 @@ __device__ __forceinline__ void adj_pass_h(const AdjArgs<T> &A, int q, const Pas
                 }
             } else {
                 const int c = a == 1 ? y : z, n = g.n[a];
+                if (!YZ) {
+#pragma unroll
+                    for (int k = 0; k < N; ++k) {
+                        contrib[k] = contrib[k] + at[k];
+                        contrib[k] = contrib[k] - up[k];
+                    }
+                    continue;
+                }
                 if (c >= 1 && old != nullptr) {
                     const int r = adj_slab_row(A.slab[0][a], c);
                     if (r >= 0) {
-                        if (a == 1) adj_slab_row_apply<T, 0, 1>(A, r, x, y, z, old, out, true, at);
-                        else adj_slab_row_apply<T, 0, 2>(A, r, x, y, z, old, out, true, at);
+                        if (a == 1) adj_slab_row_apply<I, 0, 1>(A, r, x, y, z, old, out, true, at);
+                        else adj_slab_row_apply<I, 0, 2>(A, r, x, y, z, old, out, true, at);
                     }
                 }
                 if (c + 1 <= n - 1 && old != nullptr) {
                     const int r = adj_slab_row(A.slab[0][a], c + 1);
                     if (r >= 0) {
-                        if (a == 1) adj_slab_row_apply<T, 0, 1>(A, r, x, y + 1, z, old, out, false, up);
-                        else adj_slab_row_apply<T, 0, 2>(A, r, x, y, z + 1, old, out, false, up);
+                        if (a == 1) adj_slab_row_apply<I, 0, 1>(A, r, x, y + 1, z, old, out, false, up);
+                        else adj_slab_row_apply<I, 0, 2>(A, r, x, y, z + 1, old, out, false, up);
                     }
                 }
                 const T ma = metric ? mt(a, c) : T(1), mu = metric ? mt(a, c + 1 <= n - 1 ? c + 1 : 0) : T(1);
+                if (c >= 1 && c < n - 1) {
+#pragma unroll
+                    for (int k = 0; k < N; ++k) {
+                        if (metric) {
+                            at[k] = at[k] * ma;
+                            up[k] = up[k] * mu;
+                        }
+                        contrib[k] = contrib[k] + at[k];
+                        contrib[k] = contrib[k] - up[k];
+                    }
+                    continue;
+                }
                 const bool wrap = g.periodic[a];
 #pragma unroll
                 for (int k = 0; k < N; ++k) {
@@ -391,34 +463,59 @@ __device__ __forceinline__ void adj_pass_h(const AdjArgs<T> &A, int q, const Pas
         }
         Pack<T> r;
 #pragma unroll
-        for (int k = 0; k < N; ++k) r.v[k] = x + k < nx ? hb[C].v[k] + contrib[k] : T(0);
+        for (int k = 0; k < N; ++k) r.v[k] = !last || x + k < nx ? hb[C].v[k] + contrib[k] : T(0);
         pack_store(A.hb[q ^ 1][C] + i, r);
     }
 }
 
+// Whether row (y, z) takes the YZ variant: a nonuniform mesh, a y or z face, or a slab of either family on rows c - 1 .. c + 1.
+template <typename T>
+__device__ __forceinline__ bool adj_yz(const AdjArgs<T> &A, int y, int z) {
+    const Grid<T> &g = A.g;
+    bool near = g.metric[0][0] != nullptr || g.metric[0][1] != nullptr || g.metric[0][2] != nullptr;
+#pragma unroll
+    for (int a = 1; a < 3; ++a) {
+        const int c = a == 1 ? y : z;
+        if (g.n[a] == 1) continue;
+        near = near || c == 0 || c == g.n[a] - 1;
+#pragma unroll
+        for (int f = 0; f < 2; ++f) {
+            const int *b = A.slab[f][a];
+            near = near || (c + 1 >= b[0] && c - 1 < b[1]) || (c + 1 >= b[2] && c - 1 < b[3]);
+        }
+    }
+    return near;
+}
+
+// Blocks per SM, us per launch at 200 x 200 x 80 cells, CPML 12, FP32: E pass 112 with two (128 registers), 123 with three;
+// H pass 75 with two, 60 with three. (One thread per cell: 180 and 100.) Both run below the DRAM floor's 35 and 25 us: half
+// the rows meet a slab, whose terms triple the instructions, and the E pass holds 20 input vectors per thread.
+//
 // Blocks of kPassThreads groups of one plane (blockIdx.x; plain groups first, then those near an x slab), planes on
 // blockIdx.y: ascending in the E pass, descending in the H pass. Reads parity q, writes q^1.
-template <typename T, int ACTIVE>
+template <typename T, int ACTIVE, typename I>
 __global__ void __launch_bounds__(kPassThreads, 2) k_adjoint_e(const __grid_constant__ AdjArgs<T> A, const T *__restrict__ slot, int q) {
     const unsigned p = blockIdx.x * kPassThreads + threadIdx.x;
     if (p >= A.split.total) return;
     const bool slab = p >= A.split.plain_total;
     for (int z = blockIdx.y; z < A.g.n[2]; z += gridDim.y) {
-        const PassCell<long long> w = pass_cell<long long>(A.g, A.split, p, z, slab);
-        if (slab) adj_pass_e<T, ACTIVE, true>(A, slot, q, w);
-        else adj_pass_e<T, ACTIVE, false>(A, slot, q, w);
+        const PassCell<I> w = pass_cell<I>(A.g, A.split, p, z, slab);
+        if (slab) adj_pass_e<T, ACTIVE, true, true>(A, slot, q, w);
+        else if (adj_yz(A, w.y, w.z)) adj_pass_e<T, ACTIVE, false, true>(A, slot, q, w);
+        else adj_pass_e<T, ACTIVE, false, false>(A, slot, q, w);
     }
 }
 
-template <typename T, int ACTIVE>
-__global__ void __launch_bounds__(kPassThreads, 2) k_adjoint_h(const __grid_constant__ AdjArgs<T> A, int q) {
+template <typename T, int ACTIVE, typename I>
+__global__ void __launch_bounds__(kPassThreads, sizeof(T) == 4 ? 3 : 2) k_adjoint_h(const __grid_constant__ AdjArgs<T> A, int q) {
     const unsigned p = blockIdx.x * kPassThreads + threadIdx.x;
     if (p >= A.split.total) return;
     const bool slab = p >= A.split.plain_total;
     for (int z = A.g.n[2] - 1 - (int)blockIdx.y; z >= 0; z -= gridDim.y) {
-        const PassCell<long long> w = pass_cell<long long>(A.g, A.split, p, z, slab);
-        if (slab) adj_pass_h<T, ACTIVE, true>(A, q, w);
-        else adj_pass_h<T, ACTIVE, false>(A, q, w);
+        const PassCell<I> w = pass_cell<I>(A.g, A.split, p, z, slab);
+        if (slab) adj_pass_h<T, ACTIVE, true, true>(A, q, w);
+        else if (adj_yz(A, w.y, w.z)) adj_pass_h<T, ACTIVE, false, true>(A, q, w);
+        else adj_pass_h<T, ACTIVE, false, false>(A, q, w);
     }
 }
 

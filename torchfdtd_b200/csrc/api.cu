@@ -439,7 +439,7 @@ void compute_layout(const tfd_desc *d, Layout &L) {
         L.ade[k].weight = m.weight ? b.take(std::max<size_t>(1, m.samples) * sizeof(double)) : 0;
     }
     if (tile2d_capable(d)) {
-        L.strip_rows = persist2d_eligible((long long)d->nx * d->ny) ? persist2d_strip_rows() : strip_rows((long long)d->nx * d->ny);
+        L.strip_rows = strip_rows((long long)d->nx * d->ny);
         L.tiles2d = (int)strips_of(strip_geom(d), 0, L.strip_rows).size();
         L.grid_tab = b.take(std::max(sizeof(Grid<float>), sizeof(Grid<double>)));
         L.tile_tab = b.take((size_t)L.tiles2d * sizeof(Tile2D));
@@ -487,7 +487,8 @@ struct tfd_plan {
     bool pass_metric = false, pass_wide = false;
     int pass_ctas = 0;             // > 0: all steps of a call in one launch of this many CTAs (pass_cluster: one cluster)
     bool pass_cluster = false;
-    bool two_pass = false;         // the steps run as two passes (kernel 'gather', and 'march' where two_pass_3d says so)
+    bool two_pass = false;         // the steps run as two passes (kernel 'gather', 'march' where two_pass_3d says so, 'tile2d' up to
+                                   // kPersist2dMaxCells cells that do not fit on chip)
     template <typename T> PassArgs<T> &pass();
     TfsfArgs<float> tf{};          // TFSF boxes (corrections land between and after the passes)
     TfsfArgs<double> td{};
@@ -508,7 +509,6 @@ struct tfd_plan {
     }
     int march_variant = 42;
     int tile2d_interior = 0;
-    int persist_ctas = 0;          // > 0: 2D steps run as one persistent cooperative launch of this many CTAs
     Cluster2D cluster2d{};         // ranks > 0: 2D steps run on chip in one thread-block cluster
     size_t cluster2d_smem = 0;
     std::unique_ptr<SideStream> side2d;
@@ -1803,29 +1803,6 @@ int launch_cluster2d(tfd_plan *p, int nsteps, cudaStream_t s) {
     return TFD_OK;
 }
 
-// One persistent launch of `nsteps` 2D steps with their observations (cooperative: every CTA resident).
-template <typename T>
-int launch_persist2d(tfd_plan *p, int nsteps, cudaStream_t s) {
-    const MonitorArgs<T> m = monitor_args<T>(p);
-    const int mgx = std::max(1, (p->max_samples + kMonitorThreads - 1) / kMonitorThreads), mgy = std::max(1, p->desc.n_planes);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)p->persist_ctas);
-    cfg.blockDim = dim3(k2dThreads);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    // The barrier words start every launch at zero: a launch that timed out leaves its arrival count behind.
-    TFD_CUDA(cudaMemsetAsync(p->arena + p->L.grid_bar, 0, 2 * sizeof(unsigned), s));
-    TFD_CUDA(cudaLaunchKernelEx(&cfg, k_step2d_persistent<T>, (const Grid<T> *)(p->arena + p->L.grid_tab),
-                                (const Tile2D *)(p->arena + p->L.tile_tab), p->tile2d_interior, p->L.tiles2d, m, mgx, mgy, nsteps,
-                                p->ptr<unsigned>(p->L.grid_bar)));
-    return TFD_OK;
-}
-
 // One two-pass step: the E pass, the dispersive samples, the TFSF boxes' E half step and E corrections, the H pass, the H half step and H
 // corrections (the observation launch follows in step_t).
 template <typename T>
@@ -1858,10 +1835,6 @@ template <typename T>
 int step_t(tfd_plan *p, int nsteps, cudaStream_t s) {
     if (p->kernel == TFD_KERNEL_TILE2D && p->cluster2d.ranks > 0 && !p->in_batch) {
         if (nsteps > 0) TFD_CHECK(launch_cluster2d<T>(p, nsteps, s));
-        return TFD_OK;
-    }
-    if (p->kernel == TFD_KERNEL_TILE2D && p->persist_ctas > 0 && !p->in_batch) {
-        if (nsteps > 0) TFD_CHECK(launch_persist2d<T>(p, nsteps, s));
         return TFD_OK;
     }
     if (p->two_pass && p->pass_ctas > 0) {
@@ -2066,6 +2039,10 @@ int tfd_plan_create(const tfd_desc *desc, void *arena, size_t arena_bytes, void 
         p->two_pass = p->kernel == TFD_KERNEL_GATHER || (p->kernel == TFD_KERNEL_MARCH && two_pass_3d(p));
         if (!rc && p->two_pass) rc = TFD_DISPATCH(p, setup_pass, p);
         if (!rc && tile_ok && !p->split) rc = TFD_DISPATCH(p, setup_tile2d, p, s);
+        if (!rc && p->kernel == TFD_KERNEL_TILE2D && p->cluster2d.ranks == 0 && persist2d_eligible((long long)desc->nx * desc->ny)) {
+            p->two_pass = true;
+            rc = TFD_DISPATCH(p, setup_pass, p);
+        }
     }
     if (!rc) rc = TFD_DISPATCH(p, zero_state, p, s);
     if (!rc) {
@@ -2208,7 +2185,7 @@ int tfd_step_launches(const tfd_plan *p, int32_t nsteps, int64_t *launches) {
     // Two passes: E, (dispersive samples), (TFSF E), H, (TFSF H), observation.
     long long per_step = (p->desc.n_tfsf > 0 ? 5 : 3) + ((p->desc.precision == 8 ? p->gd.ade_samples : p->gf.ade_samples) > 0);
     if (!p->two_pass && p->kernel == TFD_KERNEL_TILE2D) {
-        if ((p->persist_ctas > 0 || p->cluster2d.ranks > 0) && !p->in_batch) {
+        if (p->cluster2d.ranks > 0 && !p->in_batch) {
             *launches = nsteps > 0 ? 1 : 0;
             return TFD_OK;
         }
@@ -2645,18 +2622,22 @@ int adjoint_step_t(tfd_adjoint *adj, const void *snapshot, const void *seeds, cu
                                                                                        (const T *)seeds, adj->q);
     const dim3 grid((A.split.total + kPassThreads - 1) / kPassThreads, (unsigned)std::min(A.g.n[2], 65535));
     const T *slot = (const T *)snapshot;
+    auto both = [&](auto e, auto h) {
+        e<<<grid, kPassThreads, 0, s>>>(A, slot, adj->q);
+        h<<<grid, kPassThreads, 0, s>>>(A, adj->q);
+    };
     switch (p->desc.components) {
         case kMaskTM:
-            k_adjoint_e<T, kMaskTM><<<grid, kPassThreads, 0, s>>>(A, slot, adj->q);
-            k_adjoint_h<T, kMaskTM><<<grid, kPassThreads, 0, s>>>(A, adj->q);
+            if (p->pass_wide) both(k_adjoint_e<T, kMaskTM, long long>, k_adjoint_h<T, kMaskTM, long long>);
+            else both(k_adjoint_e<T, kMaskTM, int>, k_adjoint_h<T, kMaskTM, int>);
             break;
         case kMaskTE:
-            k_adjoint_e<T, kMaskTE><<<grid, kPassThreads, 0, s>>>(A, slot, adj->q);
-            k_adjoint_h<T, kMaskTE><<<grid, kPassThreads, 0, s>>>(A, adj->q);
+            if (p->pass_wide) both(k_adjoint_e<T, kMaskTE, long long>, k_adjoint_h<T, kMaskTE, long long>);
+            else both(k_adjoint_e<T, kMaskTE, int>, k_adjoint_h<T, kMaskTE, int>);
             break;
         default:
-            k_adjoint_e<T, kMaskAll><<<grid, kPassThreads, 0, s>>>(A, slot, adj->q);
-            k_adjoint_h<T, kMaskAll><<<grid, kPassThreads, 0, s>>>(A, adj->q);
+            if (p->pass_wide) both(k_adjoint_e<T, kMaskAll, long long>, k_adjoint_h<T, kMaskAll, long long>);
+            else both(k_adjoint_e<T, kMaskAll, int>, k_adjoint_h<T, kMaskAll, int>);
             break;
     }
     TFD_CUDA(cudaGetLastError());
