@@ -339,21 +339,15 @@ int interior_count(const std::vector<Tile2D> &t) {
 // Upper bound of the strip count of a grid for strips of at least 8 rows (two band edges add two cuts).
 int strip_capacity(int nx, int ny) { return ((nx + k2dOwnX - 1) / k2dOwnX) * ((ny + 7) / 8 + 2); }
 
-// 2D TMz grids up to this many cells step in one persistent launch (see setup_tile2d), over strips of
-// persist2d_strip_rows() rows. TFD_PERSIST2D=0/1 and TFD_PERSIST_ROWS in the environment override both,
-// for sweeps.
+// 2D TMz grids that do not fit on chip (see setup_cluster2d) and have up to this many cells run all steps of a call in one
+// launch of the two-pass kernels: us per step against per-step strip launches / strips in one cooperative launch,
+// 400 x 400: 9.4 / 16.8 / 10.9; 512 x 512: 9.2 / - / 11.7; 700 x 700: 12.6 / - / 14.5; at 1000 x 1000 the strips (15.5)
+// overtake them (15.7). TFD_PERSIST2D=0/1 in the environment overrides the size rule, for comparisons.
 constexpr long long kPersist2dMaxCells = 1LL << 19;
-constexpr int kPersist2dStripRows = 4;
 
 inline bool persist2d_eligible(long long cells) {
     const char *env = getenv("TFD_PERSIST2D");
     return env ? std::atoi(env) != 0 : cells <= kPersist2dMaxCells;
-}
-
-inline int persist2d_strip_rows() {
-    const char *env = getenv("TFD_PERSIST_ROWS");
-    const int rows = env ? std::atoi(env) : 0;
-    return rows >= 1 ? rows : kPersist2dStripRows;
 }
 
 void compute_layout(const tfd_desc *d, Layout &L) {
@@ -1233,18 +1227,6 @@ int setup_tile2d(tfd_plan *p, cudaStream_t s) {
     }
     TFD_CUDA(cudaMemcpyAsync(p->arena + p->L.grid_tab, &g, sizeof(Grid<T>), cudaMemcpyHostToDevice, s));
     TFD_CUDA(cudaMemcpyAsync(p->arena + p->L.tile_tab, tiles.data(), tiles.size() * sizeof(Tile2D), cudaMemcpyHostToDevice, s));
-    // Small grids step in one persistent launch (TFD_PERSIST2D=0/1 in the environment overrides the size
-    // rule, for sweeps): a warp per strip, and no more CTAs than can be resident together.
-    p->persist_ctas = 0;
-    if (persist2d_eligible((long long)g.n[0] * g.n[1])) {
-        int device = 0, sms = 148, per_sm = 0;
-        TFD_CUDA(cudaGetDevice(&device));
-        TFD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-        TFD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step2d_persistent<T>, k2dThreads, 0));
-        const int mblocks = std::max(1, (p->max_samples + kMonitorThreads - 1) / kMonitorThreads) * std::max(1, p->desc.n_planes);
-        const int want = std::max({1, (p->L.tiles2d + k2dWarps - 1) / k2dWarps, mblocks});
-        if (per_sm > 0) p->persist_ctas = std::min(want, per_sm * sms);
-    }
     return setup_cluster2d<T>(p);
 }
 
@@ -1743,8 +1725,9 @@ int setup_cluster2d(tfd_plan *p) {
         if (ranks > ny) continue;
         Cluster2D t{};
         t.ranks = ranks;
-        t.w = nx;
+        t.w = (nx + Pack<T>::N - 1) / Pack<T>::N * Pack<T>::N;
         t.h = ny;
+        for (int f = 0; f < 2; ++f) t.split[f] = pass_split<T>(p, f, 0);
         t.rx_e = g.rows[0][0];
         t.rx_h = g.rows[1][0];
         for (int r = 0; r <= ranks; ++r) t.r0[r] = (int)((long long)r * ny / ranks);
@@ -1755,13 +1738,16 @@ int setup_cluster2d(tfd_plan *p) {
             t.rye_max = std::max(t.rye_max, t.rye_n[r]);
             t.ryh_max = std::max(t.ryh_max, t.ryh_n[r]);
         }
+        // As many sweeps of at most kCl2dThreads threads as the largest band needs, of equal length.
+        const int groups = t.w / Pack<T>::N * t.rows_max, sweeps = (groups + kCl2dThreads - 1) / kCl2dThreads;
+        t.threads = std::max(64, ((groups + sweeps - 1) / sweeps + 31) / 32 * 32);
         const size_t bytes = (size_t)cl2d_layout(t, (int)sizeof(T)).total * sizeof(T);
-        if (bytes > (size_t)max_smem) continue;
+        if (bytes + 1024 > (size_t)max_smem) continue;    // 1 KB: the kernel's static shared memory
         TFD_CUDA(cudaFuncSetAttribute(k_step2d_cluster<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
         if (ranks > 8) TFD_CUDA(cudaFuncSetAttribute(k_step2d_cluster<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)ranks);
-        cfg.blockDim = dim3(kCl2dThreads);
+        cfg.blockDim = dim3((unsigned)t.threads);
         cfg.dynamicSmemBytes = bytes;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1788,7 +1774,7 @@ int launch_cluster2d(tfd_plan *p, int nsteps, cudaStream_t s) {
     c.count = nsteps;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)c.ranks);
-    cfg.blockDim = dim3(kCl2dThreads);
+    cfg.blockDim = dim3((unsigned)c.threads);
     cfg.dynamicSmemBytes = p->cluster2d_smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
