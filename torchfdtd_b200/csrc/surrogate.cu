@@ -833,6 +833,8 @@ struct ShiftShape {
     // K chunks of a patch lie (NP + LPAD) * 16 bytes apart: with NP a multiple of 8, the 8 (or 2) chunks of a
     // pixel that a quarter-warp stores land on distinct banks.
     static constexpr int LPAD = KC == 8 ? 1 : 4;
+    // Staging of the storing warps' rows (NC = 64: 32 rows x 64 bytes for each of the 8 warps), see stage_rows.
+    static constexpr int STAGE = NC == 64 ? 8 * 2048 : 0;
 };
 constexpr int kShiftThreads = 384;                        // 12 warps: MMA issue, 3 loading, 8 storing
 constexpr int kShiftMaxSmem = 227 * 1024;
@@ -865,6 +867,39 @@ __device__ __forceinline__ void bar_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sh_addr(bar)) : "memory");
 }
 
+// The 32 rows x 64 bytes that a storing warp holds one row per lane, moved so that four lanes write (or read) one row's 64
+// bytes: a store with one row per lane touches 32 lines for 512 bytes. buf: the warp's 2 KB, 16-byte chunks swizzled by row
+// so that both sides are free of bank conflicts. row: the lane's destination row (-1: dropped), 64 channels apart.
+__device__ __forceinline__ uint4 *stage_at(unsigned char *buf, int r, int c) {
+    return reinterpret_cast<uint4 *>(buf + r * 64 + ((c ^ ((r >> 1) & 3)) << 4));
+}
+__device__ __forceinline__ void stage_store(unsigned char *buf, int lane, const uint4 (&v)[4], long long row, bf16 *out) {
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < 4; ++c) *stage_at(buf, lane, c) = v[c];
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = 8 * i + (lane >> 2), c = lane & 3;
+        const long long to = __shfl_sync(0xffffffffu, row, r);
+        if (to >= 0) *reinterpret_cast<uint4 *>(out + to * kCo + c * 8) = *stage_at(buf, r, c);
+    }
+}
+__device__ __forceinline__ void stage_load(unsigned char *buf, int lane, uint4 (&v)[4], long long row, const bf16 *in) {
+    uint4 t[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const long long from = __shfl_sync(0xffffffffu, row, 8 * i + (lane >> 2));
+        t[i] = from >= 0 ? *reinterpret_cast<const uint4 *>(in + from * kCo + (lane & 3) * 8) : make_uint4(0, 0, 0, 0);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) *stage_at(buf, 8 * i + (lane >> 2), lane & 3) = t[i];
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < 4; ++c) v[c] = *stage_at(buf, lane, c);
+}
+
 // Warp roles: warp 0 issues the MMAs (one elected thread), warps 1-3 load patches, warps 4-11 store outputs (warp
 // 4 + q and 8 + q read tensor-memory lanes 32q..32q+31, one half of the columns each; with 16 columns warps 4-7
 // store alone). full[i]: the 96 loaders' patch of buffer i has landed (each loader waits for its own copies,
@@ -876,7 +911,8 @@ __device__ __forceinline__ void bar_arrive(uint64_t *bar) {
 template <int MODE, int CI>
 __global__ void __launch_bounds__(kShiftThreads, MODE == 0 && CI == 16 ? 3 : 1) k_conv_shift(const bf16 *__restrict__ src, const bf16 *__restrict__ wsrc,
                                                              const float *__restrict__ bias, const bf16 *__restrict__ zprev,
-                                                             bf16 *__restrict__ out0, void *__restrict__ out1, int N, int H, int W, int NB) {
+                                                             bf16 *__restrict__ out0, void *__restrict__ out1, int N, int H, int W, int NB,
+                                                             int staged) {
     using S = ShiftShape<MODE, CI>;
     constexpr int K = S::K, NC = S::NC, KC = S::KC;
     constexpr int LOADERS = 96;
@@ -897,6 +933,7 @@ __global__ void __launch_bounds__(kShiftThreads, MODE == 0 && CI == 16 ? 3 : 1) 
     uint32_t *slot = reinterpret_cast<uint32_t *>(full + 12);
     volatile int *abort = reinterpret_cast<volatile int *>(slot + 1);
     float *sbias = reinterpret_cast<float *>(full + 13);      // forward: the 64 biases
+    unsigned char *stage = reinterpret_cast<unsigned char *>(full) + 384;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tiles_img = (H * Wp + 127) / 128;
     int tend[4] = {0, 0, 0, 0}, tiles = N * tiles_img;      // MODE 2: tiles of classes 0..c
@@ -1026,7 +1063,7 @@ __global__ void __launch_bounds__(kShiftThreads, MODE == 0 && CI == 16 ? 3 : 1) 
         const int quarter = (warp - 4) & 3, cbeg = ((warp - 4) >> 2) * SPAN;
         for (int j = 0; j < count; ++j) {
             const int a = j & 1;
-            if (!bar_wait_or_abort(&accf[a], (j / 2) & 1, abort)) break;
+            if (!__all_sync(0xffffffffu, bar_wait_or_abort(&accf[a], (j / 2) & 1, abort))) break;
             tc_fence_after();
             int n, f0, c;
             decode(blockIdx.x + j * gridDim.x, n, f0, c);
@@ -1044,6 +1081,39 @@ __global__ void __launch_bounds__(kShiftThreads, MODE == 0 && CI == 16 ? 3 : 1) 
                 tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + a * NC + cbeg, v16);
 #pragma unroll
                 for (int i = 0; i < 16; ++i) vs[i] = v16[i];
+            }
+            // The accumulator is in registers: the next tile's MMAs may overwrite it.
+            tc_fence_before();
+            bar_arrive(&acce[a]);
+            if (SPAN == 32 && NC == 64 && staged) {
+                unsigned char *buf = stage + (warp - 4) * 2048;
+                const long long to = live ? row : -1;
+                uint4 q[4];
+                bf16 *qb = reinterpret_cast<bf16 *>(q);
+                if (MODE == 0) {
+                    uint4 qa[4];
+                    bf16 *ab = reinterpret_cast<bf16 *>(qa);
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) {
+                        const float z = vs[i] + sbias[cbeg + i];
+                        qb[i] = __float2bfloat16_rn(z);
+                        ab[i] = __float2bfloat16_rn(gelu(z));
+                    }
+                    stage_store(buf, lane, q, to, out0 + cbeg);
+                    stage_store(buf, lane, qa, to, reinterpret_cast<bf16 *>(out1) + cbeg);
+                } else if (zprev) {
+                    uint4 zq[4];
+                    stage_load(buf, lane, zq, to, zprev + cbeg);
+                    const bf16 *zp = reinterpret_cast<const bf16 *>(zq);
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) qb[i] = __float2bfloat16_rn(vs[i] * gelu_grad(__bfloat162float(zp[i])));
+                    stage_store(buf, lane, q, to, out0 + cbeg);
+                } else if (live) {
+                    float4 *o = reinterpret_cast<float4 *>(reinterpret_cast<float *>(out1) + row * CI + cbeg);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) o[i] = make_float4(vs[4 * i], vs[4 * i + 1], vs[4 * i + 2], vs[4 * i + 3]);
+                }
+                continue;
             }
 #pragma unroll
             for (int c0 = cbeg; c0 < cbeg + SPAN; c0 += 16) {
@@ -1078,8 +1148,6 @@ __global__ void __launch_bounds__(kShiftThreads, MODE == 0 && CI == 16 ? 3 : 1) 
                     for (int i = 0; i < 4; ++i) o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
                 }
             }
-            tc_fence_before();
-            bar_arrive(&acce[a]);
         }
     }
     tc_fence_before();
@@ -1097,9 +1165,14 @@ bool launch_shift(const bf16 *src, const bf16 *w, const float *bias, const bf16 
     const int wo = (wd - 1) / 2 + 1, wp = MODE == 2 ? wo + 1 : wd + 2;
     const long long pbytes = (long long)S::KC * ((MODE == 2 ? shift_np2(wo) : shift_np(wd)) + S::LPAD) * 16;
     int nb = 4;                          // + 384 bytes: 12 mbarriers, the tensor-memory slot, the abort flag, 64 biases
-    while (nb >= 2 && S::W_BYTES + nb * pbytes + 384 > kShiftMaxSmem) --nb;
-    if (nb < 2) return false;
-    const int smem = (int)(S::W_BYTES + nb * pbytes + 384);
+    int stage = S::STAGE;                // staged stores where two patch buffers still fit beside them
+    while (nb >= 2 && S::W_BYTES + nb * pbytes + 384 + stage > kShiftMaxSmem) --nb;
+    if (nb < 2) {
+        stage = 0;
+        nb = 2;
+        if (S::W_BYTES + nb * pbytes + 384 > kShiftMaxSmem) return false;
+    }
+    const int smem = (int)(S::W_BYTES + nb * pbytes + 384 + stage);
     static const cudaError_t attr = cudaFuncSetAttribute(k_conv_shift<MODE, CI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kShiftMaxSmem);
     (void)attr;
     static int sms = 0;
@@ -1125,7 +1198,7 @@ bool launch_shift(const bf16 *src, const bf16 *w, const float *bias, const bf16 
         for (int c = 0; c < 4; ++c) tiles += (long long)n * ((((h - (c >> 1) + 1) / 2) * wp + 127) / 128);
     }
     const long long grid = tiles < (long long)sms * per_sm ? tiles : (long long)sms * per_sm;
-    k_conv_shift<MODE, CI><<<(unsigned)grid, kShiftThreads, (size_t)smem, s>>>(src, w, bias, zprev, o0, o1, n, h, wd, nb);
+    k_conv_shift<MODE, CI><<<(unsigned)grid, kShiftThreads, (size_t)smem, s>>>(src, w, bias, zprev, o0, o1, n, h, wd, nb, stage > 0);
     return true;
 }
 
