@@ -488,7 +488,7 @@ __device__ __forceinline__ bool adj_yz(const AdjArgs<T> &A, int y, int z) {
 }
 
 // Blocks per SM, us per launch at 200 x 200 x 80 cells, CPML 12, FP32: E pass 112 with two (128 registers), 123 with three;
-// H pass 75 with two, 60 with three. (One thread per cell: 180 and 100.) Both run below the DRAM floor's 35 and 25 us: half
+// H pass 75 with two, 60 with three. (One thread per cell: 180 and 100.) Both are far from the DRAM floor of 35 and 25 us: half
 // the rows meet a slab, whose terms triple the instructions, and the E pass holds 20 input vectors per thread.
 //
 // Blocks of kPassThreads groups of one plane (blockIdx.x; plain groups first, then those near an x slab), planes on

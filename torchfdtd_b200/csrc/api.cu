@@ -340,8 +340,8 @@ int interior_count(const std::vector<Tile2D> &t) {
 int strip_capacity(int nx, int ny) { return ((nx + k2dOwnX - 1) / k2dOwnX) * ((ny + 7) / 8 + 2); }
 
 // 2D TMz grids that do not fit on chip (see setup_cluster2d) and have up to this many cells run all steps of a call in one
-// launch of the two-pass kernels: us per step against per-step strip launches / strips in one cooperative launch,
-// 400 x 400: 9.4 / 16.8 / 10.9; 512 x 512: 9.2 / - / 11.7; 700 x 700: 12.6 / - / 14.5; at 1000 x 1000 the strips (15.5)
+// launch of the two-pass kernels: us per step against strips in one cooperative launch (the earlier form),
+// 400 x 400: 9.4 / 10.9; 512 x 512: 9.2 / 11.7; 700 x 700: 12.6 / 14.5; at 1000 x 1000 the strip launches (15.5)
 // overtake them (15.7). TFD_PERSIST2D=0/1 in the environment overrides the size rule, for comparisons.
 constexpr long long kPersist2dMaxCells = 1LL << 19;
 
