@@ -253,8 +253,8 @@ int tfd_field_norm_static(const void *E, const void *H, const void *inv_eps, int
 /* Which step kernel the plan runs (enum tfd_kernel) after TFD_KERNEL_AUTO is resolved. */
 int tfd_kernel_in_use(const tfd_plan *plan, int32_t *kernel);
 
-/* How many kernel launches tfd_step(plan, nsteps) issues (small 2D TMz plans run all their steps in one
- * persistent launch; the other paths launch per step). No counterpart in the reference. */
+/* How many kernel launches tfd_step(plan, nsteps) issues: one for all steps on plans small enough to run in one cluster or
+ * cooperative launch (the two-pass step: one for every 2^20 steps), else a few per step. No counterpart in the reference. */
 int tfd_step_launches(const tfd_plan *plan, int32_t nsteps, int64_t *launches);
 
 /* ---- batches: many independent 2D TMz grids of uneven size advanced by one launch per step ----

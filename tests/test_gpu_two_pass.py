@@ -118,3 +118,14 @@ def test_reverse_step_matches_the_oracle(shape, precision, faces, component):
     got = epsilon.grad.cpu().numpy()
     assert np.linalg.norm(got - want) <= (1e-5 if precision == 'float32' else 1e-11) * np.linalg.norm(want) and np.linalg.norm(want) > 0
     model.close()
+
+
+@pytest.mark.parametrize('mode', ['1', '2'])
+def test_a_launch_runs_at_most_2_20_steps(monkeypatch, mode):
+    """The cooperative form's barrier counts every arrival of a launch in 32 bits: 2^31 - 1 steps in one launch on 148 CTAs would
+    pass 2^32 arrivals. Counted, not run."""
+    from torchfdtd_b200.native import NativeGrid
+    monkeypatch.setenv('TFD_PASS_STEPS', mode)
+    grid = NativeGrid(plan_grid(scene((13, 14, 15), 'float32')), kernel='gather')
+    assert [grid.step_launches(n) for n in (0, 1, 1 << 20, (1 << 20) + 1, 2**31 - 1)] == [0, 1, 1, 2, 2048]
+    grid.close()

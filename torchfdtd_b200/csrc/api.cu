@@ -1579,11 +1579,15 @@ int setup_pass_steps(tfd_plan *p) {
         TFD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
         TFD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass_steps_kernel<T>(p, false), kPassStepThreads, 0));
         const long long want = std::max<long long>((groups + kPassStepThreads - 1) / kPassStepThreads, mblocks);
-        if (per_sm > 0) p->pass_ctas = (int)std::min<long long>(want, (long long)sms * 1);
+        if (per_sm > 0) p->pass_ctas = (int)std::min<long long>({want, (long long)sms, 1365});      // 1365: see kPassLaunchSteps
         p->pass_cluster = false;
     }
     return TFD_OK;
 }
+
+// Steps of one launch at most: the barrier counts every arrival of a launch in 32 bits, three per step and CTA (two without
+// dispersive samples), so 2^20 steps stay below the wrap with up to 1365 CTAs.
+constexpr int kPassLaunchSteps = 1 << 20;
 
 template <typename T>
 int launch_pass_steps(tfd_plan *p, const PassArgs<T> &a, int nsteps, bool observe, cudaStream_t s) {
@@ -1593,9 +1597,15 @@ int launch_pass_steps(tfd_plan *p, const PassArgs<T> &a, int nsteps, bool observ
     cudaLaunchAttribute attr;
     pass_steps_config(cfg, attr, p->pass_cluster, p->pass_ctas, s);
     unsigned *bar = p->ptr<unsigned>(p->L.grid_bar);
-    // The barrier word starts every launch at zero: a launch that timed out leaves its arrival count behind.
-    if (!p->pass_cluster) TFD_CUDA(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), s));
-    TFD_CUDA(cudaLaunchKernelEx(&cfg, pass_steps_kernel<T>(p, p->pass_cluster), a, m, mgx, mgy, nsteps, bar));
+    PassArgs<T> launch = a;
+    while (nsteps > 0) {
+        const int count = std::min(nsteps, kPassLaunchSteps);
+        // The barrier word starts every launch at zero: a launch that timed out leaves its arrival count behind.
+        if (!p->pass_cluster) TFD_CUDA(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), s));
+        TFD_CUDA(cudaLaunchKernelEx(&cfg, pass_steps_kernel<T>(p, p->pass_cluster), launch, m, mgx, mgy, count, bar));
+        nsteps -= count;
+        if (launch.snap.base != nullptr) launch.snap.base += (long long)count * launch.snap.stride;
+    }
     return TFD_OK;
 }
 
@@ -2165,7 +2175,7 @@ int tfd_step_launches(const tfd_plan *p, int32_t nsteps, int64_t *launches) {
     if (!p || !launches) return fail(TFD_ERR_INVALID, "null argument");
     if (nsteps < 0) return fail(TFD_ERR_INVALID, "nsteps must be non-negative");
     if (p->two_pass && p->pass_ctas > 0) {
-        *launches = nsteps > 0 ? 1 : 0;
+        *launches = ((int64_t)nsteps + kPassLaunchSteps - 1) / kPassLaunchSteps;
         return TFD_OK;
     }
     // Two passes: E, (dispersive samples), (TFSF E), H, (TFSF H), observation.

@@ -551,8 +551,8 @@ __global__ void k_pass_advance(const __grid_constant__ Grid<T> g) {
 constexpr int kPassStepThreads = 512;
 constexpr int kPassWaitTries = 1 << 22;          // polls of about 0.3 us: about a second
 
-// Arrival of every CTA at barrier number `round` (0, 1, ...) of the launch; bar starts the launch at zero. False (with
-// the status recorded) when the wait runs out.
+// Arrival of every CTA at barrier number `round` (0, 1, ...) of the launch; bar starts the launch at zero and must not wrap
+// (kPassLaunchSteps in api.cu). False (with the status recorded) when the wait runs out.
 __device__ __forceinline__ bool pass_grid_barrier(unsigned *bar, unsigned round, int *status) {
     __shared__ int ok;
     __syncthreads();
