@@ -310,7 +310,8 @@ int tfd_adjoint_step(tfd_adjoint *adjoint, const void *snapshot, const void *see
  * first count - 1 steps, each leaving what its successor's transpose reads in slot 1, 2, .. of `replay` (count slots of
  * slot_bytes, at least tfd_state_bytes and a multiple of 256; slot 0 is not used, a slot is not a full restart state),
  * then transposes the count steps in reverse with `seeds` (count rows of one value per trace, or null). The replayed
- * steps record no traces or planes. Same result as load, save, step and tfd_adjoint_step one by one. */
+ * steps record no traces or planes. Same result as load, save, step and tfd_adjoint_step one by one. (A restart state holds
+ * neither the incident lines of TFSF boxes nor pole states: both ways go on from the plan's own.) */
 int tfd_adjoint_segment(tfd_adjoint *adjoint, const void *checkpoint, int32_t count, void *replay, size_t slot_bytes,
                         const void *seeds, void *stream);
 /* S in the reference layout (nx, ny, nz, 3), one value per E component (zero for components 2D does not

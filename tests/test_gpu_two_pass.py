@@ -129,3 +129,51 @@ def test_a_launch_runs_at_most_2_20_steps(monkeypatch, mode):
     grid = NativeGrid(plan_grid(scene((13, 14, 15), 'float32')), kernel='gather')
     assert [grid.step_launches(n) for n in (0, 1, 1 << 20, (1 << 20) + 1, 2**31 - 1)] == [0, 1, 1, 2, 2048]
     grid.close()
+
+
+def dispersive(project):
+    """A Drude rod through the middle of the grid."""
+    from torchfdtd_b200 import Material, Structure
+    extra = dict(materials=[Material(name='metal', model='drude', epsilon_inf=1.5, plasma_rad_s=9e15, collision_rad_s=1e14)],
+                 structures=[Structure(size=(.2, .2, project.region.size[2]), center=(.1, 0, 0), material='metal')])
+    return Project(region=project.region, sources=project.sources, monitors=project.monitors, **extra)
+
+
+@pytest.mark.parametrize('mode', ['0', '1', '2'])
+@pytest.mark.parametrize('name,precision', [('plain', 'float32'), ('tmz', 'float64'), ('dispersive', 'float64'), ('tfsf', 'float32'), ('tfsf', 'float64')])
+def test_adjoint_segment_equals_its_steps_one_by_one(monkeypatch, name, precision, mode):
+    """tfd_adjoint_segment against save, step and tfd_adjoint_step, bitwise. Both start from a reset plan: a restart state holds
+    neither a TFSF box's incident line nor pole states."""
+    import torch
+    from torchfdtd_b200.native import NativeAdjoint, NativeGrid
+    monkeypatch.setenv('TFD_PASS_STEPS', mode)
+    project = scene((21, 22, 1) if name == 'tmz' else (21, 22, 23), precision, component='Ez' if name == 'tmz' else 'Ey', steps=14)
+    if name == 'dispersive':
+        project = dispersive(project)
+    if name == 'tfsf':
+        box = Source(kind='tfsf', normal='x', direction='+', size=(.4, .4, .4), component='Ey', pulse_cycles=1, wavelength=.6)
+        project = Project(region=project.region, sources=[box], monitors=project.monitors)
+    plan = plan_grid(project)
+    assert bool(plan.tfsf) == (name == 'tfsf')
+    grid = NativeGrid(plan, kernel='gather')
+    adjoint = NativeAdjoint(grid)
+    count = 12
+    seeds = torch.tensor(np.random.default_rng(5).normal(size=(count, 1)), dtype=grid.torch_dtype, device='cuda')
+    slots = torch.zeros((count, grid.state_bytes()), dtype=torch.uint8, device='cuda')
+    replay, checkpoint = torch.zeros_like(slots), torch.zeros_like(slots[0])
+    grid.reset()
+    grid.save_state(checkpoint)
+    for j in range(count):
+        grid.save_state(slots[j])
+        grid.step(1)
+    for j in range(count - 1, -1, -1):
+        adjoint.step(slots[j], seeds[j].contiguous())
+    want = adjoint.sensitivity().clone()
+    grid.reset()
+    adjoint.reset()
+    adjoint.segment(checkpoint, count, replay, seeds)
+    got = adjoint.sensitivity()
+    assert want.abs().max() > 0
+    np.testing.assert_array_equal(got.cpu().numpy(), want.cpu().numpy())
+    adjoint.close()
+    grid.close()

@@ -2643,6 +2643,7 @@ int adjoint_step_t(tfd_adjoint *adj, const void *snapshot, const void *seeds, cu
 
 // Restores the checkpoint of a segment of `count` steps, replays all but the last step (each leaving its H and E-family
 // CPML memories in its slot of `replay`) and transposes the steps in reverse. The checkpoint is the first step's snapshot.
+// With TFSF boxes the corrections of H land after the H pass: a slot is then saved whole after the step.
 template <typename T>
 int adjoint_segment_t(tfd_adjoint *adj, const char *checkpoint, int count, char *replay, size_t slot_bytes, const T *seeds, cudaStream_t s) {
     tfd_plan *p = adj->p;
@@ -2654,14 +2655,16 @@ int adjoint_segment_t(tfd_adjoint *adj, const char *checkpoint, int count, char 
     for (int c = 0; c < 3; ++c) a.snap.sH[c] = A.sH[c];
     for (int ax = 0; ax < 3; ++ax)
         for (int j = 0; j < 2; ++j) a.snap.sPsiE[ax][j] = A.sPsiE[ax][j];
+    const bool whole = p->desc.n_tfsf > 0;
     if (p->pass_ctas > 0 && count > 1) {
         a.snap.base = (T *)(replay + slot_bytes);
         TFD_CHECK(launch_pass_steps<T>(p, a, count - 1, false, s));
     } else {
         for (int j = 1; j < count; ++j) {
-            a.snap.base = (T *)(replay + j * slot_bytes);
+            if (!whole) a.snap.base = (T *)(replay + j * slot_bytes);
             TFD_CHECK(launch_two_pass<T>(p, a, s));
             k_pass_advance<T><<<1, 1, 0, s>>>(a.g);
+            if (whole) TFD_CHECK(state_copy_t<T>(p, replay + j * slot_bytes, true, s));
         }
     }
     for (int j = count - 1; j >= 0; --j)
