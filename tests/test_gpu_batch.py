@@ -284,3 +284,23 @@ def test_batch_accepts_per_case_epsilon():
     report = run_tensor_batch(projects, epsilon=eps)
     for p, e, item in zip(projects, eps, report.items):
         assert_results_equal(item.result, Simulation(p, epsilon=e).run(kernel='tile2d'))
+
+
+@pytest.mark.parametrize('precision', ['float32', 'float64'])
+def test_on_chip_plan_steps_after_a_smaller_plan_was_created(precision):
+    """The shared-memory limit of the on-chip kernel covers every plan alive, not the one created last."""
+    from torchfdtd_b200.models import Source
+    def plan_of(nx, ny):
+        return plan_grid(Project(region=Region(dimension='2d', size=(nx * .05, ny * .05, 1), mesh=.05, pml_cells=8, steps=12,
+                                               precision=precision, backend='cuda'),
+                                 sources=[Source(center=(.1, 0, 0), component='Ez', pulse_cycles=1, wavelength=.6)]))
+    large, small = plan_of(180, 170), plan_of(40, 36)
+    a, b = native(large, 'tile2d'), native(small, 'tile2d')
+    for grid, plan in ((a, large), (b, small)):
+        assert grid.step_launches(5) == 1
+        grid.step(plan.steps)
+        oracle = YeeOracle(plan).run()
+        E, H = grid.get_fields()
+        np.testing.assert_array_equal(E, oracle.E)
+        np.testing.assert_array_equal(H, oracle.H)
+        grid.close()

@@ -1752,8 +1752,10 @@ int setup_cluster2d(tfd_plan *p) {
         const int groups = t.w / Pack<T>::N * t.rows_max, sweeps = (groups + kCl2dThreads - 1) / kCl2dThreads;
         t.threads = std::max(64, ((groups + sweeps - 1) / sweeps + 31) / 32 * 32);
         const size_t bytes = (size_t)cl2d_layout(t, (int)sizeof(T)).total * sizeof(T);
-        if (bytes + 1024 > (size_t)max_smem) continue;    // 1 KB: the kernel's static shared memory
-        TFD_CUDA(cudaFuncSetAttribute(k_step2d_cluster<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        const int limit = max_smem - 1024;                // 1 KB: the kernel's static shared memory
+        if (bytes > (size_t)limit) continue;
+        // The limit belongs to the kernel, not to the plan: always the largest, whatever this plan takes of it.
+        TFD_CUDA(cudaFuncSetAttribute(k_step2d_cluster<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
         if (ranks > 8) TFD_CUDA(cudaFuncSetAttribute(k_step2d_cluster<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)ranks);
