@@ -250,7 +250,9 @@ int tfd_device_status(tfd_plan *plan, int32_t *status, void *stream);
 int tfd_field_norm_static(const void *E, const void *H, const void *inv_eps, int64_t cells, int32_t material_samples,
                           int32_t precision, double *out, void *stream);
 
-/* Which step kernel the plan runs (enum tfd_kernel) after TFD_KERNEL_AUTO is resolved. */
+/* Which step kernel the plan runs (enum tfd_kernel) after TFD_KERNEL_AUTO is resolved. TFD_KERNEL_GATHER: the two-pass step
+ * (most 3D plans); TFD_KERNEL_MARCH: the marching kernel (the largest uniform FP32 ones, or asked for by name);
+ * TFD_KERNEL_TILE2D: the 2D TMz forms (on chip, all steps of a call in one launch, or strips per step, by size). */
 int tfd_kernel_in_use(const tfd_plan *plan, int32_t *kernel);
 
 /* How many kernel launches tfd_step(plan, nsteps) issues: one for all steps on plans small enough to run in one cluster or

@@ -133,19 +133,21 @@ def test_float32_against_float64_runs_of_the_same_kernels():
     assert max(v for v in out['strip'].values()) < 1e-5
 
 
+@pytest.mark.parametrize('kernel,runs', [('march', 'march'), ('auto', 'gather')])
 @pytest.mark.parametrize('precision', ['float32', 'float64'])
-def test_graded_mesh_306x306x172_metric_mixed_launch_every_memory(precision):
+def test_graded_mesh_306x306x172_metric_mixed_launch_every_memory(precision, kernel, runs):
     """The graded-mesh workload (metric equidistribution, auto-refined box, physically graded CPML) for 10 steps
-    through the metric mixed march launch: the pure body with metric factors on the interior block, the general
-    metric body elsewhere; fields, every CPML memory and the traces bitwise against the C oracle."""
+    through the metric mixed march launch (the pure body with metric factors on the interior block, the general
+    metric body elsewhere) and through the default, the two-pass step; fields, every CPML memory and the traces
+    bitwise against the C oracle."""
     from torchfdtd_b200.native import NativeGrid
     project, eps = config_project('graded', 10, precision)
     plan = plan_grid(project)
     if eps is not None:
         plan.epsilon, plan.inv_eps = eps, (1 / eps).astype(plan.dtype)
     assert plan.metrics, 'the workload must run on a nonuniform mesh'
-    grid = NativeGrid(plan)
-    assert grid.kernel == 'march'
+    grid = NativeGrid(plan, kernel=kernel)
+    assert grid.kernel == runs
     grid.step(10)
     E, H = grid.get_fields()
     psi = grid.get_psi()

@@ -42,7 +42,7 @@ def skip_unmarchable(plan_or_project, kernel):
     if kernel != 'gather' and project is not None and (
             any(s.enabled and s.kind == 'tfsf' for s in project.sources)
             or any(m.oscillators for m in project.materials if m.name in {s.material for s in project.structures if s.enabled})):
-        pytest.skip('TFSF and dispersive scenes run the split gather kernels')
+        pytest.skip('TFSF and dispersive scenes run the two-pass step')
     periodic_xy = any(region.boundaries.pair(a)[0].kind == 'periodic' for a in (0, 1))
     if kernel == 'march' and region.dimension == '2d':
         pytest.skip('scene runs the gather kernel')

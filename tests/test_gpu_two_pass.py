@@ -85,7 +85,7 @@ def test_default_3d_step_equals_the_marching_kernel(shape, steps):
     out = []
     for variant in (0, 14):
         grid = NativeGrid(plan, variant=variant)
-        assert grid.kernel == 'march'
+        assert grid.kernel == ('march' if variant else 'gather')
         grid.set_fields(*start)
         grid.step(steps)
         out.append((*grid.get_fields(), *grid.get_psi()))
@@ -177,3 +177,24 @@ def test_adjoint_segment_equals_its_steps_one_by_one(monkeypatch, name, precisio
     np.testing.assert_array_equal(got.cpu().numpy(), want.cpu().numpy())
     adjoint.close()
     grid.close()
+
+
+def test_kernel_name_is_the_kernel_that_steps(monkeypatch):
+    """NativeGrid.kernel and the launches of a step: a kernel asked for by name runs, 'auto' names its choice ('tile2d': any of
+    the 2D TMz forms)."""
+    from torchfdtd_b200.native import NativeGrid
+    flat = scene((48, 44, 1), 'float32', component='Ez')
+    monkeypatch.setenv('TFD_PASS_STEPS', '0')
+    got = []
+    for project, kernel, env in ((scene((21, 18, 16), 'float32'), 'auto', {}), (scene((21, 18, 16), 'float32'), 'march', {}),
+                                 (scene((21, 18, 16), 'float64'), 'march', {}), (flat, 'auto', {}),
+                                 (flat, 'tile2d', {'TFD_CLUSTER2D': '0'}), (flat, 'tile2d', {'TFD_CLUSTER2D': '0', 'TFD_PERSIST2D': '0'})):
+        for k in ('TFD_CLUSTER2D', 'TFD_PERSIST2D'):
+            monkeypatch.delenv(k, raising=False)
+        for k, v in env.items():
+            monkeypatch.setenv(k, v)
+        grid = NativeGrid(plan_grid(project), kernel=kernel)
+        got.append((grid.kernel, grid.step_launches(4)))
+        grid.close()
+    assert [k for k, _ in got] == ['gather', 'march', 'march', 'tile2d', 'tile2d', 'tile2d']
+    assert got[0][1] == 12 and got[3][1] == 1 and got[4][1] == 12 and all(n <= 12 for _, n in got)

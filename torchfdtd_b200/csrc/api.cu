@@ -1613,11 +1613,11 @@ int launch_pass_steps(tfd_plan *p, const PassArgs<T> &a, int nsteps, bool observ
 // against 76, but needs the largest grids to get there; measured, us per step (two-pass / march): 160 x 120 x 40: 27 /
 // 43; 192^3: 136 / 207; 256^3: 281 / 398; 320^3: 514 / 647; 400^3: 971 / 1018; 512 x 512 x 256: 960-990 / 907. With
 // periodic x / y faces (512 x 512 x 128: 465 / 626), a nonuniform mesh (306 x 306 x 176: 314 / 379) or in FP64 (151 x 133 x
-// 117, periodic: 89 / 222) the marching kernel runs slower bodies and the two passes win at every size tried. An
-// explicit launch variant (or TFD_MARCH_VARIANT) asks for the marching kernel.
+// 117, periodic: 89 / 222) the marching kernel runs slower bodies and the two passes win at every size tried. Kernel
+// 'march' by name, an explicit launch variant or TFD_MARCH_VARIANT asks for the marching kernel.
 bool two_pass_3d(const tfd_plan *p) {
     const tfd_desc &d = p->desc;
-    if (d.launch_variant != 0 || getenv("TFD_MARCH_VARIANT")) return false;
+    if (d.kernel == TFD_KERNEL_MARCH || d.launch_variant != 0 || getenv("TFD_MARCH_VARIANT")) return false;
     const bool seams = d.face[0][0] == TFD_FACE_PERIODIC || d.face[1][0] == TFD_FACE_PERIODIC;
     return d.precision == 8 || p->march_metric || seams || (long long)d.nx * d.ny * d.nz < kMarchMinCells;
 }
@@ -2169,7 +2169,7 @@ int tfd_device_status(tfd_plan *p, int32_t *status, void *stream) {
 
 int tfd_kernel_in_use(const tfd_plan *p, int32_t *kernel) {
     if (!p || !kernel) return fail(TFD_ERR_INVALID, "null argument");
-    *kernel = p->kernel;
+    *kernel = p->two_pass && p->kernel == TFD_KERNEL_MARCH ? TFD_KERNEL_GATHER : p->kernel;
     return TFD_OK;
 }
 

@@ -468,7 +468,8 @@ class Simulation:
         return plan, eps
 
     def run(self, progress=None, cancel=None, cuda_graph=True, cuda_graph_steps=1, kernel='auto', launch=None):
-        """``kernel``: 'auto' (the marching kernel for 3D, the tile kernel for 2D TMz, else gather) or a name.
+        """``kernel``: 'auto' (3D: the two-pass step, 'gather', or the marching kernel, by size; 2D TMz:
+        'tile2d'; else gather) or a name.
         ``launch``: None (default launch shape), an explicit launch variant, or 'auto' to measure the
         marching kernel's variants on scratch plans first (``tuning.select_launch``; cached per process)."""
         with ENGINE_LOCK:
@@ -509,9 +510,10 @@ class Simulation:
             variant, tuning = 0, None
             if launch == 'auto':
                 if plan.dimension == '3d' and kernel in ('auto', 'march'):
-                    from .tuning import select_launch
+                    from .tuning import grid_candidates, select_launch
                     try:
-                        tuning = select_launch(plan)
+                        # Variant 0 is the default of kernel 'auto'; the marching kernel's own default is among its variants.
+                        tuning = select_launch(plan, None if kernel == 'auto' else [v for v in grid_candidates(plan) if v])
                         variant = tuning.choice
                     except ValueError as exc:          # too few steps to tune, or no marching kernel for this scene
                         tuning = dict(skipped=str(exc))

@@ -94,7 +94,8 @@ def grid_candidates(plan):
 
 
 def select_launch(plan, candidates=None, *, steps=8, repeats=5, device=None):
-    """Measure marching-kernel launch variants for ``plan`` (a 3D ``GridPlan``) and return a ``LaunchTuning``.
+    """Measure the default step (variant 0, kernel 'auto') and the marching kernel's launch variants for ``plan`` (a 3D
+    ``GridPlan``) and return a ``LaunchTuning``.
 
     Scratch plans are created per candidate (all at once when device memory allows, else one candidate at a
     time with the same number of sweeps). Results are cached per (GPU, plan shape, CPML layout, candidates)."""
@@ -104,6 +105,8 @@ def select_launch(plan, candidates=None, *, steps=8, repeats=5, device=None):
         raise ValueError('select_launch tunes the 3D marching kernel; 2D batches use tune_tensor_batch.')
     if isinstance(repeats, bool) or not isinstance(repeats, int) or repeats < 1:
         raise ValueError('repeats must be a positive integer.')
+    if plan.tfsf or plan.ade:                            # the marching kernel refuses them
+        raise ValueError('No launch variant is supported for this plan.')
     device = torch.device('cuda', torch.cuda.current_device() if device is None else device)
     candidates = list(dict.fromkeys(candidates or grid_candidates(plan)))
     steps = min(steps, plan.steps // (repeats + 1))      # scratch runs stay within the plan's own steps
@@ -121,7 +124,7 @@ def select_launch(plan, candidates=None, *, steps=8, repeats=5, device=None):
     with torch.cuda.device(device), torch.cuda.stream(stream):
         for v in candidates:
             try:
-                grids[v] = NativeGrid(plan, kernel='march', variant=v)
+                grids[v] = NativeGrid(plan, kernel='march' if v else 'auto', variant=v)
             except ValueError as exc:
                 records.append(dict(variant=v, status='unsupported', reason=str(exc)))
                 continue
@@ -138,7 +141,7 @@ def select_launch(plan, candidates=None, *, steps=8, repeats=5, device=None):
         else:
             samples, digests = {}, {}
             for v in grids:
-                g = NativeGrid(plan, kernel='march', variant=v)
+                g = NativeGrid(plan, kernel='march' if v else 'auto', variant=v)
                 samples.update(_interleaved({v: lambda n: g.step(n, stream)}, repeats, steps, stream))
                 digests[v] = _digest(g.get_fields())
                 g.close()
