@@ -198,3 +198,26 @@ def test_kernel_name_is_the_kernel_that_steps(monkeypatch):
         grid.close()
     assert [k for k, _ in got] == ['gather', 'march', 'march', 'tile2d', 'tile2d', 'tile2d']
     assert got[0][1] == 12 and got[3][1] == 1 and got[4][1] == 12 and all(n <= 12 for _, n in got)
+
+
+@pytest.mark.parametrize('mode', ['0', '1', '2'])
+@pytest.mark.parametrize('shape,precision,frequencies', [((21, 18, 16), 'float32', 1), ((21, 18, 16), 'float64', 7), ((40, 36, 1), 'float32', 257)])
+def test_plane_accumulators_of_any_frequency_count(monkeypatch, shape, precision, frequencies, mode):
+    """DFT planes of the one-launch forms and of a launch per step, below, at and past the chunks of frequencies that one
+    pass over the accumulators takes; the double-precision sums of the CPU oracle to 1e-12."""
+    from oracle.cpu import CpuOracle
+    from torchfdtd_b200 import FieldMonitor, SpectrumSettings
+    from torchfdtd_b200.native import NativeGrid
+    monkeypatch.setenv('TFD_PASS_STEPS', mode)
+    project = scene(shape, precision, component='Hz' if shape[2] == 1 else 'Ey', steps=13)
+    spectrum = SpectrumSettings(sampling='frequency', frequency_points=frequencies, apodization='none')
+    plane = FieldMonitor(normal='x', center=(.1, 0, 0), size=(0, .3, 1 if shape[2] == 1 else .2), dft_precision='float64', spectrum=spectrum)
+    plan = plan_grid(Project(region=project.region, sources=project.sources, monitors=[plane]))
+    want = CpuOracle(plan).run_with_planes(dft_float64=True)
+    grid = NativeGrid(plan, kernel='gather')
+    grid.step(6)
+    grid.step(7)
+    got = grid.get_plane(0)
+    assert got.shape[0] == frequencies and np.abs(got).max() > 0
+    assert np.linalg.norm(got - want[0]) <= 1e-12 * np.linalg.norm(want[0])
+    grid.close()

@@ -83,15 +83,32 @@ __device__ __forceinline__ void monitor_work(const MonitorArgs<T> &m, int bx, in
         }
         __syncthreads();
         if (live) {
-            for (int f = 0; f < nf; ++f) {
-                const double2 ph = magnetic ? phase_h[f] : phase_e[f];
-                double *acc = pl.acc + 2 * (((long long)(f0 + f) * pl.points + p) * pl.components + c);
-                acc[0] += ph.x * value;
-                acc[1] += ph.y * value;
+            // Four accumulators in flight: one at a time cost a memory round trip per frequency (0.27 us; a plane of 17,472
+            // samples and 200 frequencies, 160 x 120 x 40 cells: 147 us per step against 77 in three launches).
+            constexpr int B = 4;
+            const long long stride = (long long)pl.points * pl.components;
+            double2 *acc = reinterpret_cast<double2 *>(pl.acc) + (long long)f0 * stride + s;
+            for (int f = 0; f < nf; f += B) {
+                double2 a[B];
+#pragma unroll
+                for (int j = 0; j < B; ++j)
+                    if (f + j < nf) a[j] = acc[(f + j) * stride];
+#pragma unroll
+                for (int j = 0; j < B; ++j)
+                    if (f + j < nf) {
+                        const double2 ph = magnetic ? phase_h[f + j] : phase_e[f + j];
+                        a[j].x += ph.x * value;
+                        a[j].y += ph.y * value;
+                        acc[(f + j) * stride] = a[j];
+                    }
             }
         }
     }
 }
+
+// The same as a call: k_pass_steps would spill for its registers.
+template <typename T>
+__device__ __noinline__ void monitor_call(const MonitorArgs<T> &m, int bx, int by, long long n, int gx) { monitor_work(m, bx, by, n, gx); }
 
 // The last block of a launch to finish advances the step counter; every block read it first.
 __device__ __forceinline__ void finish_step(long long *counter, unsigned *done, long long n) {

@@ -596,7 +596,7 @@ __global__ void __launch_bounds__(kPassStepThreads, 1) k_pass_steps(const __grid
         const int par = (int)(n & 1);
         T *slot = A.snap.base != nullptr ? A.snap.base + k * A.snap.stride : nullptr;
         if (k > 0)
-            for (int b = blockIdx.x; b < mgx * mgy; b += gridDim.x) monitor_work(m, b % mgx, b / mgx, n - 1, mgx);
+            for (int b = blockIdx.x; b < mgx * mgy; b += gridDim.x) monitor_call(m, b % mgx, b / mgx, n - 1, mgx);
         for (int it = blockIdx.x; it < items; it += gridDim.x)
             pass_block_e<T, ACTIVE, METRIC, ADE, int>(A, (it % per_plane) * kPassStepThreads + threadIdx.x, it / per_plane, par, n, slot);
         if (!barrier()) return;
@@ -609,7 +609,7 @@ __global__ void __launch_bounds__(kPassStepThreads, 1) k_pass_steps(const __grid
         if (!barrier()) return;
     }
     if (n > n0)
-        for (int b = blockIdx.x; b < mgx * mgy; b += gridDim.x) monitor_work(m, b % mgx, b / mgx, n - 1, mgx);
+        for (int b = blockIdx.x; b < mgx * mgy; b += gridDim.x) monitor_call(m, b % mgx, b / mgx, n - 1, mgx);
     if (blockIdx.x == 0 && threadIdx.x == 0) *g.counter = n;
 }
 
