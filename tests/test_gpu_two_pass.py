@@ -197,7 +197,7 @@ def test_kernel_name_is_the_kernel_that_steps(monkeypatch):
         got.append((grid.kernel, grid.step_launches(4)))
         grid.close()
     assert [k for k, _ in got] == ['gather', 'march', 'march', 'tile2d', 'tile2d', 'tile2d']
-    assert got[0][1] == 12 and got[3][1] == 1 and got[4][1] == 12 and all(n <= 12 for _, n in got)
+    assert got[0][1] == 8 and got[3][1] == 1 and got[4][1] == 8 and all(n <= 12 for _, n in got)
 
 
 @pytest.mark.parametrize('mode', ['0', '1', '2'])
@@ -220,4 +220,37 @@ def test_plane_accumulators_of_any_frequency_count(monkeypatch, shape, precision
     got = grid.get_plane(0)
     assert got.shape[0] == frequencies and np.abs(got).max() > 0
     assert np.linalg.norm(got - want[0]) <= 1e-12 * np.linalg.norm(want[0])
+    grid.close()
+
+
+@pytest.mark.parametrize('shape,precision,plane', [
+    ((21, 18, 16), 'float32', False), ((21, 18, 16), 'float64', True), ((42, 37, 30), 'float32', False), ((42, 37, 30), 'float32', True),
+    ((70, 66, 72), 'float32', True), ((90, 100, 103), 'float64', False), ((103, 90, 1), 'float32', True), ((103, 90, 1), 'float64', True)])
+def test_calls_of_any_length_match_the_oracle(shape, precision, plane):
+    """The default launch form of short and long calls on one plan: one cluster, one cooperative launch of one, two (moved on
+    from sweep to sweep) and more than six sweeps, strips in one launch, launches per pass."""
+    from oracle.cpu import CpuOracle
+    from torchfdtd_b200 import FieldMonitor, SpectrumSettings
+    from torchfdtd_b200.native import NativeGrid
+    two_d = shape[2] == 1
+    project = scene(shape, precision, component='Ez' if two_d else 'Ey', steps=14)
+    if plane:
+        spectrum = SpectrumSettings(sampling='frequency', frequency_points=3, apodization='none')
+        monitor = FieldMonitor(normal='y', center=(0, .1, 0), size=(.4, 0, 1 if two_d else .2), dft_precision='float64', spectrum=spectrum)
+        project = Project(region=project.region, sources=project.sources, monitors=[*project.monitors, monitor])
+    plan = plan_grid(project)
+    oracle = CpuOracle(plan)
+    grid = NativeGrid(plan)
+    want = oracle.run_with_planes(dft_float64=True)
+    for count in (1, 4, 2, 3, 20):
+        grid.step(count)
+    E, H = grid.get_fields()
+    np.testing.assert_array_equal(E, oracle.E)
+    np.testing.assert_array_equal(H, oracle.H)
+    np.testing.assert_array_equal(grid.get_traces(), oracle.traces)
+    for got, expected in zip(grid.get_psi(), oracle.memory_states):
+        np.testing.assert_array_equal(got, expected)
+    for k, value in enumerate(want):
+        assert np.linalg.norm(grid.get_plane(k) - value) <= 1e-12 * np.linalg.norm(value) and np.linalg.norm(value) > 0
+    assert grid.counter() == plan.steps and grid.device_status() == 0
     grid.close()

@@ -339,10 +339,41 @@ int interior_count(const std::vector<Tile2D> &t) {
 // Upper bound of the strip count of a grid for strips of at least 8 rows (two band edges add two cuts).
 int strip_capacity(int nx, int ny) { return ((nx + k2dOwnX - 1) / k2dOwnX) * ((ny + 7) / 8 + 2); }
 
+// Steps in one launch (k_pass_steps), us per step in calls of 48 steps (FP32, CPML 5 unless stated):
+// - one cluster while a pass is one group per thread of its 16 CTAs and the plan has no DFT plane: TE, 200 x 121 cells: 6.9,
+//   cooperative 8.0, two launches per step 9.7; 24^3 cells: 12.5 / 13.7 / 16.2. With a plane its work delays every step of the
+//   cluster, while the cooperative form leaves it to SMs without groups: 30^3 cells, 1,944 samples: 19.8 / 14.9 / 22.1;
+// - the cooperative form up to kPassFewSweeps sweeps of its CTAs: 60^3: 16.7 against 20.3 in launches; 160 x 120 x 40: 19.7 / 25.1;
+//   120^3: 41.9 / 49.7 (CPML 12: 51.5 / 50.7); 130^3, 8 sweeps: 64.9 / 63.7. In FP64 both forms run 512 threads per SM and the
+//   line lies at kPassGridGroups64: 128^3: 86.9 / 92.3; 140^3: 106 / 118;
+// - launches where the samples of the planes outnumber the cooperative form's threads: 160 x 120 x 40 cells with 147,408 samples of
+//   20 frequencies: 57.1 / 50.3; with 17,472 of 200: 74 / 79.
+// Calls of fewer than kPassMany steps (a captured single step is how Simulation.run replays) do not earn the cooperative launch's
+// 5-7 us back: 60^3 cells, one step: 22.6 against 21.3; TE, 350 x 300: 14.5 / 12.5. The cluster's does not cost them: TE, 200 x 121: 10.4 /
+// 11.4, while its observations are light (630 samples of 20 frequencies: 16.4 / 18.6; of 200: 39.1 / 33).
+constexpr int kPassClusterRanks = 16;
+constexpr long long kPassClusterGroups = (long long)kPassClusterRanks * kPassStepThreads, kPassFewSweeps = 6;
+constexpr long long kPassGridGroups = kPassFewSweeps * 148 * kPassStepThreads, kPassGridGroups64 = 3LL << 19;
+constexpr long long kPassLightSums = 1LL << 15;           // accumulators
+constexpr int kPassMany = 4;
+
+// Steps of one launch at most: the barrier counts every arrival of a launch in 32 bits, three per step and CTA (two without
+// dispersive samples), so 2^20 steps stay below the wrap with up to 1365 CTAs.
+constexpr int kPassLaunchSteps = 1 << 20;
+
+// Threads of a CTA: `groups` shared evenly by the fewest sweeps that `ctas` CTAs of at most kPassStepThreads threads need, so that a
+// grid of few groups gets small CTAs on many SMs (30^3 cells: 113 of 64 threads, 14 us per step; 15 of 512 threads took 23).
+// More than kPassFewSweeps sweeps: full CTAs (FP64, 128 x 120 x 100 cells: 69 us against 77 with 480 threads).
+int pass_steps_threads(long long groups, int ctas) {
+    const long long full = (long long)ctas * kPassStepThreads, sweeps = (groups + full - 1) / full;
+    if (sweeps > kPassFewSweeps) return kPassStepThreads;
+    const long long even = (groups + ctas * sweeps - 1) / (ctas * sweeps);
+    return (int)std::max<long long>(64, (even + 31) / 32 * 32);
+}
+
 // 2D TMz grids that do not fit on chip (see setup_cluster2d) and have up to this many cells run all steps of a call in one
-// launch of the two-pass kernels: us per step against strips in one cooperative launch (the earlier form),
-// 400 x 400: 9.4 / 10.9; 512 x 512: 9.2 / 11.7; 700 x 700: 12.6 / 14.5; at 1000 x 1000 the strip launches (15.5)
-// overtake them (15.7). TFD_PERSIST2D=0/1 in the environment overrides the size rule, for comparisons.
+// launch of the two-pass kernels: us per step against strips in one cooperative launch (the earlier form), 512 x 512: 9.2 / 11.7; 700 x 700: 12.6 / 14.5; at 1000 x 1000 the strip launches (15.5) overtake them
+// (15.7). TFD_PERSIST2D=0 in the environment asks for a launch per step, 1 for one launch whatever the size, for comparisons.
 constexpr long long kPersist2dMaxCells = 1LL << 19;
 
 inline bool persist2d_eligible(long long cells) {
@@ -458,6 +489,10 @@ namespace tfd {
 void set_error(const std::string &msg) { g_error = msg; }
 }  // namespace tfd
 
+// One launch for all two-pass steps of a call: CTAs (0: a launch per pass instead), threads of each, one cluster or a
+// cooperative launch, and the chunks (PassArgs).
+struct PassShape { int ctas, threads; bool cluster; unsigned chunks, rotate; };
+
 struct tfd_plan {
     tfd_desc desc;               // sizes and flags only; host pointers are not kept
     Layout L;
@@ -479,8 +514,7 @@ struct tfd_plan {
     PassArgs<float> pf;            // two-pass step (kernel 'gather')
     PassArgs<double> pd;
     bool pass_metric = false, pass_wide = false;
-    int pass_ctas = 0;             // > 0: all steps of a call in one launch of this many CTAs (pass_cluster: one cluster)
-    bool pass_cluster = false;
+    PassShape pass_many{}, pass_few{};   // two-pass steps of a call in one launch: calls of kPassMany steps and more, shorter ones
     bool two_pass = false;         // the steps run as two passes (kernel 'gather', 'march' where two_pass_3d says so, 'tile2d' up to
                                    // kPersist2dMaxCells cells that do not fit on chip)
     template <typename T> PassArgs<T> &pass();
@@ -1525,21 +1559,29 @@ PassSteps<T> pass_steps_kernel(tfd_plan *p, bool cluster) {
 }
 
 constexpr long long kMarchMinCells = 1LL << 26;      // see two_pass_3d
-// Steps in one launch (k_pass_steps): one cluster while a pass is one group per thread of its 16 CTAs (a 200 x 121 TE grid:
-// 7.1 us per step, 9.3 with the grid barrier, 11.0 with three launches per step), the grid barrier up to kPassGridGroups
-// (320 x 240 cells: 8.8 us against 10.7 in the cluster and 10.8; 160 x 120 x 40 cells: 27.0 against 32.0; but 192^3 cells,
-// 1.8 M groups: 147 against 136) or three times that in FP64, where both forms run 512 threads per SM (151 x 133 x 117
-// cells, 1.2 M groups: 91 against 102).
-constexpr int kPassClusterRanks = 16;
-constexpr long long kPassClusterGroups = (long long)kPassClusterRanks * kPassStepThreads, kPassGridGroups = 1LL << 19;
+// A plane's chunks end with its x-slab groups, the slow ones. Moved on by `rotate` CTAs from sweep to sweep, a CTA's chunks
+// lie 1 / sweeps of a plane apart, so that all CTAs meet slab groups about equally often: 100^3 cells 33.7 -> 30.0 us per step,
+// 110^3 40.0 -> 32.6, 120^3 47.9 -> 40.9. Over many sweeps the chunks mix by themselves (FP64, 140^3: 105 us, 111 when rotated).
+unsigned pass_steps_rotation(long long total, long long groups, int ctas, int threads) {
+    const double chunks = (double)total / threads;
+    const long long sweeps = (groups + (long long)ctas * threads - 1) / ((long long)ctas * threads);
+    if (sweeps < 2 || sweeps > kPassFewSweeps || chunks <= 1) return 0;
+    unsigned best = 0;
+    double least = 1;
+    for (int r = 0; r < ctas && r <= 2 * chunks; ++r) {
+        const double turns = (ctas + r) / chunks, off = std::fabs(turns - std::floor(turns) - 1.0 / sweeps);
+        if (off < least) { least = off; best = r; }
+    }
+    return best;
+}
 
-inline void pass_steps_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &attr, bool cluster, int ctas, cudaStream_t s) {
-    cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3(kPassStepThreads);
+inline void pass_steps_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &attr, const PassShape &shape, cudaStream_t s) {
+    cfg.gridDim = dim3((unsigned)shape.ctas);
+    cfg.blockDim = dim3((unsigned)shape.threads);
     cfg.stream = s;
-    if (cluster) {
+    if (shape.cluster) {
         attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = (unsigned)ctas;
+        attr.val.clusterDim.x = (unsigned)shape.ctas;
         attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     } else {
         attr.id = cudaLaunchAttributeCooperative;
@@ -1549,60 +1591,79 @@ inline void pass_steps_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &attr
     cfg.numAttrs = 1;
 }
 
-// Whether the plan's steps run in one launch, and on how many CTAs.
+// The launch forms of the plan's steps. TFD_PASS_STEPS in the environment (0: a launch per pass, 1: one cluster, 2: one
+// cooperative launch) overrides the rules, for comparisons.
 template <typename T>
 int setup_pass_steps(tfd_plan *p) {
     const PassArgs<T> &a = p->pass<T>();
-    p->pass_ctas = 0;
+    p->pass_many = p->pass_few = PassShape{};
     const char *env = getenv("TFD_PASS_STEPS");
     const int mode = env ? std::atoi(env) : -1;
     if (p->pass_wide || p->desc.n_tfsf > 0 || mode == 0) return TFD_OK;
     const long long groups = (long long)a.split[0].total * a.g.n[2];
-    const int mblocks = std::max(1, (p->max_samples + kPassStepThreads - 1) / kPassStepThreads) * std::max(1, p->desc.n_planes);
+    long long samples = 0, sums = 0;                      // DFT samples, and their accumulators
+    for (int k = 0; k < p->desc.n_planes; ++k) {
+        const long long n = (long long)p->planes_p[k] * p->planes_c[k];
+        samples += n;
+        sums += n * p->planes_f[k];
+    }
+    PassShape cluster{}, grid{};
     if (mode == 1 || (mode < 0 && groups <= kPassClusterGroups)) {
         PassSteps<T> kernel = pass_steps_kernel<T>(p, true);
+        // One CTA stays clear of groups for the observations where the others have the threads.
+        const int busy = groups <= (long long)(kPassClusterRanks - 1) * kPassStepThreads ? kPassClusterRanks - 1 : kPassClusterRanks;
+        cluster = PassShape{kPassClusterRanks, pass_steps_threads(groups, busy), true};
+        cluster.chunks = (unsigned)((groups + cluster.threads - 1) / cluster.threads);
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr;
-        pass_steps_config(cfg, attr, true, kPassClusterRanks, nullptr);
+        pass_steps_config(cfg, attr, cluster, nullptr);
         int clusters = 0;
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-            cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters >= 1) {
-            p->pass_ctas = kPassClusterRanks;
-            p->pass_cluster = true;
-            return TFD_OK;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters < 1) {
+            cudaGetLastError();
+            cluster = PassShape{};
         }
-        cudaGetLastError();
     }
-    if (mode == 2 || (mode < 0 && groups <= kPassGridGroups * (sizeof(T) == 8 ? 3 : 1))) {
+    if (mode == 2 || (mode < 0 && groups <= (sizeof(T) == 8 ? kPassGridGroups64 : kPassGridGroups))) {
         int device = 0, sms = 148, per_sm = 0;
         TFD_CUDA(cudaGetDevice(&device));
         TFD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-        TFD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass_steps_kernel<T>(p, false), kPassStepThreads, 0));
-        const long long want = std::max<long long>((groups + kPassStepThreads - 1) / kPassStepThreads, mblocks);
-        if (per_sm > 0) p->pass_ctas = (int)std::min<long long>({want, (long long)sms, 1365});      // 1365: see kPassLaunchSteps
-        p->pass_cluster = false;
+        const int ctas = std::min(sms, 1365);             // 1365: see kPassLaunchSteps
+        grid.threads = pass_steps_threads(groups, ctas);
+        TFD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass_steps_kernel<T>(p, false), grid.threads, 0));
+        // CTAs for the groups and, while there are SMs left, others for the observations.
+        const long long mblocks = (long long)std::max(1, (p->max_samples + grid.threads - 1) / grid.threads) * std::max(1, p->desc.n_planes);
+        const long long want = (groups + grid.threads - 1) / grid.threads + mblocks;
+        if (per_sm > 0) grid.ctas = (int)std::min<long long>(want, ctas);
+        grid.chunks = (unsigned)((groups + grid.threads - 1) / grid.threads);
+        grid.rotate = pass_steps_rotation(a.split[0].total, groups, grid.ctas, grid.threads);
     }
+    if (mode >= 0) {
+        p->pass_many = p->pass_few = mode == 1 ? cluster : grid;
+        return TFD_OK;
+    }
+    if (samples == 0) p->pass_many = cluster.ctas > 0 ? cluster : grid;
+    else if (samples <= (long long)grid.ctas * grid.threads) p->pass_many = grid;
+    if (sums <= kPassLightSums) p->pass_few = cluster;
     return TFD_OK;
 }
 
-// Steps of one launch at most: the barrier counts every arrival of a launch in 32 bits, three per step and CTA (two without
-// dispersive samples), so 2^20 steps stay below the wrap with up to 1365 CTAs.
-constexpr int kPassLaunchSteps = 1 << 20;
-
 template <typename T>
-int launch_pass_steps(tfd_plan *p, const PassArgs<T> &a, int nsteps, bool observe, cudaStream_t s) {
+int launch_pass_steps(tfd_plan *p, const PassShape &shape, const PassArgs<T> &a, int nsteps, bool observe, cudaStream_t s) {
     const MonitorArgs<T> m = monitor_args<T>(p);
-    const int mgx = observe ? std::max(1, (p->max_samples + kPassStepThreads - 1) / kPassStepThreads) : 0, mgy = std::max(1, p->desc.n_planes);
+    const int mgx = observe ? std::max(1, (p->max_samples + shape.threads - 1) / shape.threads) : 0, mgy = std::max(1, p->desc.n_planes);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr;
-    pass_steps_config(cfg, attr, p->pass_cluster, p->pass_ctas, s);
+    pass_steps_config(cfg, attr, shape, s);
     unsigned *bar = p->ptr<unsigned>(p->L.grid_bar);
     PassArgs<T> launch = a;
+    launch.chunks = shape.chunks;
+    launch.rotate = shape.rotate;
     while (nsteps > 0) {
         const int count = std::min(nsteps, kPassLaunchSteps);
         // The barrier word starts every launch at zero: a launch that timed out leaves its arrival count behind.
-        if (!p->pass_cluster) TFD_CUDA(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), s));
-        TFD_CUDA(cudaLaunchKernelEx(&cfg, pass_steps_kernel<T>(p, p->pass_cluster), launch, m, mgx, mgy, count, bar));
+        if (!shape.cluster) TFD_CUDA(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), s));
+        TFD_CUDA(cudaLaunchKernelEx(&cfg, pass_steps_kernel<T>(p, shape.cluster), launch, m, mgx, mgy, count, bar));
         nsteps -= count;
         if (launch.snap.base != nullptr) launch.snap.base += (long long)count * launch.snap.stride;
     }
@@ -1622,6 +1683,9 @@ bool two_pass_3d(const tfd_plan *p) {
     return d.precision == 8 || p->march_metric || seams || (long long)d.nx * d.ny * d.nz < kMarchMinCells;
 }
 
+// The multiplier that pass_divide takes for a division by d.
+unsigned pass_magic(unsigned d) { return d <= 1 ? 0xffffffffu : (unsigned)(((1ull << 32) + d - 1) / d); }
+
 // The groups of a row apart from the x slabs of family f (f < 0: of both), widened by `reach` cells.
 template <typename T>
 PassSplit pass_split(const tfd_plan *p, int f, int reach) {
@@ -1638,10 +1702,9 @@ PassSplit pass_split(const tfd_plan *p, int f, int reach) {
         if (e - x > sp.plain) { sp.x_lo = x; sp.plain = e - x; }
         x = std::max(x, e);
     }
-    auto magic = [](int d) { return d <= 1 ? 0xffffffffu : (unsigned)(((1ull << 32) + d - 1) / d); };
     sp.slab = groups - sp.plain;
-    sp.magic_plain = magic(sp.plain);
-    sp.magic_slab = magic(sp.slab);
+    sp.magic_plain = pass_magic(sp.plain);
+    sp.magic_slab = pass_magic(sp.slab);
     sp.plain_total = (unsigned)sp.plain * p->desc.ny;
     sp.total = (unsigned)groups * p->desc.ny;
     return sp;
@@ -1658,6 +1721,7 @@ int setup_pass(tfd_plan *p) {
     for (size_t q = 0; q < p->seg_f.size(); ++q) a.tables |= ++count[p->seg_f[q]][p->seg_a[q]] > 2;
     if (!a.tables) TFD_CHECK(slab_bounds(p, a.slab));
     for (int f = 0; f < 2; ++f) a.split[f] = pass_split<T>(p, f, 0);
+    a.magic_total = pass_magic(a.split[0].total);
     p->pass_metric = false;
     for (int f = 0; f < 2; ++f)
         for (int ax = 0; ax < 3; ++ax) {
@@ -1667,18 +1731,34 @@ int setup_pass(tfd_plan *p) {
     return setup_pass_steps<T>(p);
 }
 
-// One pass (E, or H from the stored E_new) of the two-pass step. Arrays of 2^31 elements and more take the variant with
-// 64-bit indices, which handles every other feature at run time.
+dim3 pass_blocks(const tfd_plan *p, unsigned total) {
+    return dim3((total + kPassThreads - 1) / kPassThreads, (unsigned)std::min(p->desc.nz, 65535));
+}
+
+// Whether the H pass ends the step (k_pass_h), point traces included: no planes, no boxes, few traces (one block records them)
+// and few blocks. us per captured step with a third launch / without: TE, 400 x 400 cells, 157 blocks: 10.5 / 8.9; 700 x 700, 480: 14.7 /
+// 13.7; 1000 x 1000, 977: 17.3 / 18.3; 60^3 cells, 240: 20.5 / 20.2; FP64 128^3, 4,096: 91 / 106.
+constexpr long long kPassEndBlocks = 512;
+constexpr int kPassEndTraces = 1024;
+
+template <typename T>
+bool pass_ends_step(tfd_plan *p) {
+    const dim3 b = pass_blocks(p, p->pass<T>().split[1].total);
+    return p->desc.n_planes == 0 && p->desc.n_tfsf == 0 && p->desc.n_traces <= kPassEndTraces && (long long)b.x * b.y <= kPassEndBlocks;
+}
+
+// One pass (E, or H from the stored E_new; end: the H pass ends the step) of the two-pass step. Arrays of 2^31 elements and more
+// take the variant with 64-bit indices, which handles every other feature at run time.
 template <typename T, int ACTIVE>
-void launch_pass_active(tfd_plan *p, const PassArgs<T> &a, bool h, cudaStream_t s) {
-    const dim3 grid((a.split[0].total + kPassThreads - 1) / kPassThreads, (unsigned)std::min(a.g.n[2], 65535));
+void launch_pass_active(tfd_plan *p, const PassArgs<T> &a, bool h, const MonitorArgs<T> &m, int end, cudaStream_t s) {
+    const dim3 grid = pass_blocks(p, a.split[0].total);
     const bool ade = a.g.ade_map[0] != nullptr;          // soft sources on dispersive samples
     if (p->pass_wide) {
-        if (h) k_pass_h<T, ACTIVE, true, long long><<<grid, kPassThreads, 0, s>>>(a);
+        if (h) k_pass_h<T, ACTIVE, true, long long><<<grid, kPassThreads, 0, s>>>(a, m, end);
         else k_pass_e<T, ACTIVE, true, true, long long><<<grid, kPassThreads, 0, s>>>(a);
     } else if (h) {
-        if (p->pass_metric) k_pass_h<T, ACTIVE, true, int><<<grid, kPassThreads, 0, s>>>(a);
-        else k_pass_h<T, ACTIVE, false, int><<<grid, kPassThreads, 0, s>>>(a);
+        if (p->pass_metric) k_pass_h<T, ACTIVE, true, int><<<grid, kPassThreads, 0, s>>>(a, m, end);
+        else k_pass_h<T, ACTIVE, false, int><<<grid, kPassThreads, 0, s>>>(a, m, end);
     } else if (ade) {
         if (p->pass_metric) k_pass_e<T, ACTIVE, true, true, int><<<grid, kPassThreads, 0, s>>>(a);
         else k_pass_e<T, ACTIVE, false, true, int><<<grid, kPassThreads, 0, s>>>(a);
@@ -1689,11 +1769,11 @@ void launch_pass_active(tfd_plan *p, const PassArgs<T> &a, bool h, cudaStream_t 
 }
 
 template <typename T>
-void launch_pass(tfd_plan *p, const PassArgs<T> &a, bool h, cudaStream_t s) {
+void launch_pass(tfd_plan *p, const PassArgs<T> &a, bool h, const MonitorArgs<T> &m, int end, cudaStream_t s) {
     switch (p->grid<T>().active) {
-        case kMaskTM: launch_pass_active<T, kMaskTM>(p, a, h, s); break;
-        case kMaskTE: launch_pass_active<T, kMaskTE>(p, a, h, s); break;
-        default: launch_pass_active<T, kMaskAll>(p, a, h, s); break;
+        case kMaskTM: launch_pass_active<T, kMaskTM>(p, a, h, m, end, s); break;
+        case kMaskTE: launch_pass_active<T, kMaskTE>(p, a, h, m, end, s); break;
+        default: launch_pass_active<T, kMaskAll>(p, a, h, m, end, s); break;
     }
 }
 
@@ -1802,14 +1882,14 @@ int launch_cluster2d(tfd_plan *p, int nsteps, cudaStream_t s) {
 }
 
 // One two-pass step: the E pass, the dispersive samples, the TFSF boxes' E half step and E corrections, the H pass, the H half step and H
-// corrections (the observation launch follows in step_t).
+// corrections. Unless the H pass ends the step, the observation launch (step_t) or k_pass_advance follows.
 template <typename T>
-int launch_two_pass(tfd_plan *p, const PassArgs<T> &pass, cudaStream_t s) {
-    launch_pass<T>(p, pass, false, s);
+int launch_two_pass(tfd_plan *p, const PassArgs<T> &pass, const MonitorArgs<T> &m, int end, cudaStream_t s) {
+    launch_pass<T>(p, pass, false, m, 0, s);
     const int samples = p->grid<T>().ade_samples;
     if (samples > 0) k_pass_ade<T><<<(samples + kPassThreads - 1) / kPassThreads, kPassThreads, 0, s>>>(p->pass<T>().g, samples);
     if (p->desc.n_tfsf == 0) {
-        launch_pass<T>(p, pass, true, s);
+        launch_pass<T>(p, pass, true, m, end, s);
         return TFD_OK;
     }
     const Grid<T> &g = p->grid<T>();
@@ -1824,7 +1904,7 @@ int launch_two_pass(tfd_plan *p, const PassArgs<T> &pass, cudaStream_t s) {
     for (int k = 0; k < a.boxes; ++k) longest = std::max(longest, a.box[k].count + std::max(a.box[k].n[0], a.box[k].n[1]));
     const dim3 tgrid((unsigned)((longest + kTfsfThreads - 1) / kTfsfThreads), (unsigned)a.boxes);
     k_tfsf<T><<<tgrid, kTfsfThreads, 0, s>>>(a, 0);
-    launch_pass<T>(p, pass, true, s);
+    launch_pass<T>(p, pass, true, m, 0, s);
     k_tfsf<T><<<tgrid, kTfsfThreads, 0, s>>>(a, 1);
     return TFD_OK;
 }
@@ -1835,15 +1915,15 @@ int step_t(tfd_plan *p, int nsteps, cudaStream_t s) {
         if (nsteps > 0) TFD_CHECK(launch_cluster2d<T>(p, nsteps, s));
         return TFD_OK;
     }
-    if (p->two_pass && p->pass_ctas > 0) {
-        if (nsteps > 0) TFD_CHECK(launch_pass_steps<T>(p, p->pass<T>(), nsteps, true, s));
-        return TFD_OK;
-    }
+    const PassShape &shape = nsteps < kPassMany ? p->pass_few : p->pass_many;
+    if (p->two_pass && shape.ctas > 0) return launch_pass_steps<T>(p, shape, p->pass<T>(), nsteps, true, s);
+    const int end = p->two_pass && pass_ends_step<T>(p);
     const MonitorArgs<T> m = monitor_args<T>(p);
     dim3 mgrid((unsigned)std::max(1, (p->max_samples + kMonitorThreads - 1) / kMonitorThreads), (unsigned)std::max(1, p->desc.n_planes));
     for (int k = 0; k < nsteps; ++k) {
         if (p->two_pass) {
-            TFD_CHECK(launch_two_pass<T>(p, p->pass<T>(), s));
+            TFD_CHECK(launch_two_pass<T>(p, p->pass<T>(), m, end, s));
+            if (end) continue;
         } else if (p->kernel == TFD_KERNEL_MARCH) {
             launch_march_any<T>(p, s);
         } else {
@@ -2176,12 +2256,14 @@ int tfd_kernel_in_use(const tfd_plan *p, int32_t *kernel) {
 int tfd_step_launches(const tfd_plan *p, int32_t nsteps, int64_t *launches) {
     if (!p || !launches) return fail(TFD_ERR_INVALID, "null argument");
     if (nsteps < 0) return fail(TFD_ERR_INVALID, "nsteps must be non-negative");
-    if (p->two_pass && p->pass_ctas > 0) {
+    if (p->two_pass && (nsteps < kPassMany ? p->pass_few : p->pass_many).ctas > 0) {
         *launches = ((int64_t)nsteps + kPassLaunchSteps - 1) / kPassLaunchSteps;
         return TFD_OK;
     }
-    // Two passes: E, (dispersive samples), (TFSF E), H, (TFSF H), observation.
-    long long per_step = (p->desc.n_tfsf > 0 ? 5 : 3) + ((p->desc.precision == 8 ? p->gd.ade_samples : p->gf.ade_samples) > 0);
+    // Two passes: E, (dispersive samples), (TFSF E), H, (TFSF H), (observation).
+    tfd_plan *q = const_cast<tfd_plan *>(p);
+    long long per_step = (p->desc.n_tfsf > 0 ? 5 : 3) + ((p->desc.precision == 8 ? p->gd.ade_samples : p->gf.ade_samples) > 0) -
+                         (p->two_pass && TFD_DISPATCH(q, pass_ends_step, q) ? 1 : 0);
     if (!p->two_pass && p->kernel == TFD_KERNEL_TILE2D) {
         if (p->cluster2d.ranks > 0 && !p->in_batch) {
             *launches = nsteps > 0 ? 1 : 0;
@@ -2657,14 +2739,15 @@ int adjoint_segment_t(tfd_adjoint *adj, const char *checkpoint, int count, char 
     for (int c = 0; c < 3; ++c) a.snap.sH[c] = A.sH[c];
     for (int ax = 0; ax < 3; ++ax)
         for (int j = 0; j < 2; ++j) a.snap.sPsiE[ax][j] = A.sPsiE[ax][j];
+    const MonitorArgs<T> m = monitor_args<T>(p);
     const bool whole = p->desc.n_tfsf > 0;
-    if (p->pass_ctas > 0 && count > 1) {
+    if (p->pass_many.ctas > 0 && count > 1) {
         a.snap.base = (T *)(replay + slot_bytes);
-        TFD_CHECK(launch_pass_steps<T>(p, a, count - 1, false, s));
+        TFD_CHECK(launch_pass_steps<T>(p, p->pass_many, a, count - 1, false, s));
     } else {
         for (int j = 1; j < count; ++j) {
             if (!whole) a.snap.base = (T *)(replay + j * slot_bytes);
-            TFD_CHECK(launch_two_pass<T>(p, a, s));
+            TFD_CHECK(launch_two_pass<T>(p, a, m, 0, s));
             k_pass_advance<T><<<1, 1, 0, s>>>(a.g);
             if (whole) TFD_CHECK(state_copy_t<T>(p, replay + j * slot_bytes, true, s));
         }

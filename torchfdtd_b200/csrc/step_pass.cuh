@@ -57,6 +57,9 @@ struct PassArgs {
     int slab[2][3][4];           // per family and axis: lo0, hi0, lo1, hi1 of the two CPML slabs
     int tables;                  // 1: more than two slabs on some axis, slab rows come from the row tables
     PassSplit split[2];          // per family
+    // k_pass_steps (PassShape in api.cu): chunks of blockDim.x groups, numbered through the planes (magic_total divides a group's
+    // number by split[].total); rotate: CTAs that the chunks move on by from sweep to sweep.
+    unsigned chunks, magic_total, rotate;
     PassSnap<T> snap;
 };
 
@@ -528,12 +531,36 @@ __global__ void __launch_bounds__(kPassThreads, kPassBlocks<T>) k_pass_e(const _
         pass_block_e<T, ACTIVE, METRIC, ADE, I>(A, blockIdx.x * kPassThreads + threadIdx.x, z, (int)(n & 1), n, A.snap.base);
 }
 
+// end: nothing follows in the step but point traces, which the block that finishes last records before it advances the step
+// counter. A third launch costs 1-2 us on small grids (captured TE steps, 400 x 400 cells: 10.5 us with it, 8.9 without); with
+// many blocks their fences cost more than that (1000 x 1000: 17.3 and 18.3), see pass_ends_step in api.cu.
 template <typename T, int ACTIVE, bool METRIC, typename I>
-__global__ void __launch_bounds__(kPassThreads, kPassBlocks<T>) k_pass_h(const __grid_constant__ PassArgs<T> A) {
+__global__ void __launch_bounds__(kPassThreads, kPassBlocks<T>) k_pass_h(const __grid_constant__ PassArgs<T> A,
+                                                                        const __grid_constant__ MonitorArgs<T> m, int end) {
     const long long n = *A.g.counter;
     if (n >= A.g.steps) return;
     for (int z = A.g.n[2] - 1 - (int)blockIdx.y; z >= 0; z -= gridDim.y)
         pass_block_h<T, ACTIVE, METRIC, I>(A, blockIdx.x * kPassThreads + threadIdx.x, z, (int)(n & 1), n, A.snap.base);
+    if (!end) return;
+    __shared__ int is_last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        is_last = atomicAdd(m.done, 1u) == gridDim.x * gridDim.y - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!is_last) return;
+    const long long shift = ((n + 1) & 1) ? m.count : 0;
+    for (int k = threadIdx.x; k < m.n_traces; k += kPassThreads) {
+        const TraceDev t = m.traces[k];
+        const T *base = m.field[3 * t.family + t.comp];
+        m.trace_out[n * m.n_traces + k] = base ? __ldcg(base + shift + t.offset) : T(0);
+    }
+    if (threadIdx.x == 0) {
+        *m.done = 0;
+        *A.g.counter = n + 1;
+    }
 }
 
 // The step counter alone (a replayed step records no observations).
@@ -545,9 +572,10 @@ __global__ void k_pass_advance(const __grid_constant__ Grid<T> g) {
 
 // ---- many steps in one launch ----------------------------------------------------------------------------------
 // Grids whose passes are shorter than a launch (a 200 x 121 TE step: three launches of 3 us each for 24,200 cells)
-// run all steps of a tfd_step call in one cooperative launch: E pass, barrier, H pass, barrier, the observations of
-// step n - 1 taken beside the E pass of step n (they read the parity that step n leaves alone). CLUSTER: one
-// thread-block cluster, hardware barrier; else every SM one CTA and a counting barrier in global memory.
+// run all steps of a tfd_step call in one launch: E pass, barrier, H pass, barrier, the observations of step n - 1 taken
+// beside the E pass of step n (they read the parity that step n leaves alone). CLUSTER: one thread-block cluster, hardware
+// barrier; else at most one CTA per SM and a counting barrier in global memory. The groups are shared out evenly, a chunk per CTA
+// and sweep; the observations start on the CTAs with the fewest chunks.
 constexpr int kPassStepThreads = 512;
 constexpr int kPassWaitTries = 1 << 22;          // polls of about 0.3 us: about a second
 
@@ -580,7 +608,41 @@ __global__ void __launch_bounds__(kPassStepThreads, 1) k_pass_steps(const __grid
                                                                     int mgx, int mgy, int count, unsigned *bar) {
     const Grid<T> &g = A.g;
     const long long n0 = *g.counter;
-    const int per_plane = (int)((A.split[0].total + kPassStepThreads - 1) / kPassStepThreads), items = per_plane * g.n[2];
+    // This thread's group p of plane z in the chunk at CTA position c of a sweep, and the position in the next sweep. FP32 steps
+    // from sweep to sweep (on_p groups and on_z planes on; [1]: where c + rotate passes the last CTA); in FP64 the registers for
+    // that spill (151 x 133 x 117 cells: 3 % longer), and each chunk divides.
+    constexpr bool STEPPED = sizeof(T) == 4;
+    const unsigned total = A.split[0].total;
+    int p0;
+    const int z0 = pass_divide(blockIdx.x * blockDim.x + threadIdx.x, total, A.magic_total, p0);
+    unsigned on_p[2], on_z[2];
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+        const unsigned by = (A.rotate + (d == 0 ? gridDim.x : 0)) * blockDim.x;
+        on_z[d] = by / total;
+        on_p[d] = by - on_z[d] * total;
+    }
+    auto at = [&](unsigned chunk, unsigned &p, unsigned &z) {
+        if (STEPPED) return;
+        int rest;
+        z = (unsigned)pass_divide(chunk * blockDim.x + threadIdx.x, total, A.magic_total, rest);
+        p = (unsigned)rest;
+    };
+    auto next = [&](unsigned &c, unsigned &p, unsigned &z) {
+        c += A.rotate;
+        const int d = c >= gridDim.x;
+        if (d) c -= gridDim.x;
+        if (!STEPPED) return;
+        p += d ? on_p[1] : on_p[0];
+        z += d ? on_z[1] : on_z[0];
+        if (p >= total) {
+            p -= total;
+            ++z;
+        }
+    };
+    // The observations: first on the CTAs at the end of the last sweep, which may have no chunk in it.
+    const unsigned sweeps = (A.chunks + gridDim.x - 1) / gridDim.x;
+    const int last = (int)(gridDim.x - 1 - (blockIdx.x + (sweeps - 1) * A.rotate) % gridDim.x);
     unsigned round = 0;
     auto barrier = [&]() -> bool {
         if constexpr (CLUSTER) {
@@ -596,20 +658,24 @@ __global__ void __launch_bounds__(kPassStepThreads, 1) k_pass_steps(const __grid
         const int par = (int)(n & 1);
         T *slot = A.snap.base != nullptr ? A.snap.base + k * A.snap.stride : nullptr;
         if (k > 0)
-            for (int b = blockIdx.x; b < mgx * mgy; b += gridDim.x) monitor_call(m, b % mgx, b / mgx, n - 1, mgx);
-        for (int it = blockIdx.x; it < items; it += gridDim.x)
-            pass_block_e<T, ACTIVE, METRIC, ADE, int>(A, (it % per_plane) * kPassStepThreads + threadIdx.x, it / per_plane, par, n, slot);
+            for (int b = last; b < mgx * mgy; b += gridDim.x) monitor_call(m, b % mgx, b / mgx, n - 1, mgx);
+        for (unsigned sweep = 0, c = blockIdx.x, p = p0, z = z0; sweep < A.chunks; sweep += gridDim.x, next(c, p, z)) {
+            at(sweep + c, p, z);
+            if (sweep + c < A.chunks && z < (unsigned)g.n[2]) pass_block_e<T, ACTIVE, METRIC, ADE, int>(A, p, (int)z, par, n, slot);
+        }
         if (!barrier()) return;
         if (ADE) {
-            for (int j = blockIdx.x * kPassStepThreads + threadIdx.x; j < g.ade_samples; j += gridDim.x * kPassStepThreads) pass_ade(g, j, par, n);
+            for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < g.ade_samples; j += gridDim.x * blockDim.x) pass_ade(g, j, par, n);
             if (!barrier()) return;
         }
-        for (int it = blockIdx.x; it < items; it += gridDim.x)
-            pass_block_h<T, ACTIVE, METRIC, int>(A, (it % per_plane) * kPassStepThreads + threadIdx.x, it / per_plane, par, n, slot);
+        for (unsigned sweep = 0, c = blockIdx.x, p = p0, z = z0; sweep < A.chunks; sweep += gridDim.x, next(c, p, z)) {
+            at(sweep + c, p, z);
+            if (sweep + c < A.chunks && z < (unsigned)g.n[2]) pass_block_h<T, ACTIVE, METRIC, int>(A, p, (int)z, par, n, slot);
+        }
         if (!barrier()) return;
     }
     if (n > n0)
-        for (int b = blockIdx.x; b < mgx * mgy; b += gridDim.x) monitor_call(m, b % mgx, b / mgx, n - 1, mgx);
+        for (int b = last; b < mgx * mgy; b += gridDim.x) monitor_call(m, b % mgx, b / mgx, n - 1, mgx);
     if (blockIdx.x == 0 && threadIdx.x == 0) *g.counter = n;
 }
 
