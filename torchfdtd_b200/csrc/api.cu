@@ -113,6 +113,7 @@ struct Layout {
     size_t check = 0;              // tfd_set_permittivity / tfd_field_check results
     size_t grid_tab = 0, tile_tab = 0;   // 2D tile kernel: this plan's Grid struct and its tile table
     int tiles2d = 0, strip_rows = 8;
+    bool persist_strips = false;   // all steps of a call over strips in one launch
     size_t stage_bytes = 0;
     size_t psi_total = 0;          // elements of the reference psi vector
     size_t total = 0;
@@ -372,13 +373,30 @@ int pass_steps_threads(long long groups, int ctas) {
 }
 
 // 2D TMz grids that do not fit on chip (see setup_cluster2d) and have up to this many cells run all steps of a call in one
-// launch of the two-pass kernels: us per step against strips in one cooperative launch (the earlier form), 512 x 512: 9.2 / 11.7; 700 x 700: 12.6 / 14.5; at 1000 x 1000 the strip launches (15.5) overtake them
+// launch of the two-pass kernels: us per step against strips in one cooperative launch, without DFT planes (with them:
+// persist_strips), 512 x 512: 9.2 / 11.7; 700 x 700: 12.6 / 14.5; at 1000 x 1000 the strip launches (15.5) overtake them
 // (15.7). TFD_PERSIST2D=0 in the environment asks for a launch per step, 1 for one launch whatever the size, for comparisons.
 constexpr long long kPersist2dMaxCells = 1LL << 19;
 
 inline bool persist2d_eligible(long long cells) {
     const char *env = getenv("TFD_PERSIST2D");
     return env ? std::atoi(env) != 0 : cells <= kPersist2dMaxCells;
+}
+
+// With DFT planes, which keep a plan off chip, FP32 grids step over strips of kPersistStripRows rows in that launch: one grid
+// barrier per step instead of two. us per step against the two passes, one plane and one frequency: 64 x 64 cells: 10.4 / 8.6;
+// 150 x 140: 8.8 / 9.3; 300 x 200: 8.5 / 9.6; 350 x 300: 8.8 / 9.9; 400 x 400: 12.0 / 8.7; 512 x 512: 11.3 / 12.1 (20 frequencies: 11.8
+// / 14.1). Past kPersistStripCells the two passes win only while CTAs are left for the observations (400 x 400, not 512 x 512).
+constexpr int kPersistStripRows = 4;
+constexpr long long kPersistStripMinCells = 1LL << 13, kPersistStripCells = 1LL << 17;
+
+inline bool persist_strips(const tfd_desc *d) {
+    const long long cells = (long long)d->nx * d->ny;
+    if (d->n_planes == 0 || d->precision != 4 || cells < kPersistStripMinCells || !persist2d_eligible(cells)) return false;
+    long long samples = 0;
+    for (int k = 0; k < d->n_planes; ++k) samples += (long long)d->planes[k].points * d->planes[k].components;
+    const long long groups = (long long)((d->nx + 3) / 4) * d->ny;
+    return cells <= kPersistStripCells || groups + samples > 148LL * pass_steps_threads(groups, 148);
 }
 
 void compute_layout(const tfd_desc *d, Layout &L) {
@@ -464,7 +482,8 @@ void compute_layout(const tfd_desc *d, Layout &L) {
         L.ade[k].weight = m.weight ? b.take(std::max<size_t>(1, m.samples) * sizeof(double)) : 0;
     }
     if (tile2d_capable(d)) {
-        L.strip_rows = strip_rows((long long)d->nx * d->ny);
+        L.persist_strips = persist_strips(d);
+        L.strip_rows = L.persist_strips ? kPersistStripRows : strip_rows((long long)d->nx * d->ny);
         L.tiles2d = (int)strips_of(strip_geom(d), 0, L.strip_rows).size();
         L.grid_tab = b.take(std::max(sizeof(Grid<float>), sizeof(Grid<double>)));
         L.tile_tab = b.take((size_t)L.tiles2d * sizeof(Tile2D));
@@ -515,6 +534,7 @@ struct tfd_plan {
     PassArgs<double> pd;
     bool pass_metric = false, pass_wide = false;
     PassShape pass_many{}, pass_few{};   // two-pass steps of a call in one launch: calls of kPassMany steps and more, shorter ones
+    int persist_ctas = 0;          // > 0: 2D TMz steps over strips in one cooperative launch of this many CTAs
     bool two_pass = false;         // the steps run as two passes (kernel 'gather', 'march' where two_pass_3d says so, 'tile2d' up to
                                    // kPersist2dMaxCells cells that do not fit on chip)
     template <typename T> PassArgs<T> &pass();
@@ -1261,6 +1281,16 @@ int setup_tile2d(tfd_plan *p, cudaStream_t s) {
     }
     TFD_CUDA(cudaMemcpyAsync(p->arena + p->L.grid_tab, &g, sizeof(Grid<T>), cudaMemcpyHostToDevice, s));
     TFD_CUDA(cudaMemcpyAsync(p->arena + p->L.tile_tab, tiles.data(), tiles.size() * sizeof(Tile2D), cudaMemcpyHostToDevice, s));
+    p->persist_ctas = 0;
+    if (p->L.persist_strips) {                       // a warp per strip, and no more CTAs than can be resident together
+        int device = 0, sms = 148, per_sm = 0;
+        TFD_CUDA(cudaGetDevice(&device));
+        TFD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+        TFD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step2d_persistent<T>, k2dThreads, 0));
+        const int mblocks = std::max(1, (p->max_samples + kMonitorThreads - 1) / kMonitorThreads) * std::max(1, p->desc.n_planes);
+        const int want = std::max({1, (p->L.tiles2d + k2dWarps - 1) / k2dWarps, mblocks});
+        p->persist_ctas = std::min(want, per_sm * sms);
+    }
     return setup_cluster2d<T>(p);
 }
 
@@ -1881,6 +1911,28 @@ int launch_cluster2d(tfd_plan *p, int nsteps, cudaStream_t s) {
     return TFD_OK;
 }
 
+// One launch of `nsteps` 2D steps over strips with their observations (cooperative: every CTA resident).
+template <typename T>
+int launch_persist2d(tfd_plan *p, int nsteps, cudaStream_t s) {
+    const MonitorArgs<T> m = monitor_args<T>(p);
+    const int mgx = std::max(1, (p->max_samples + kMonitorThreads - 1) / kMonitorThreads), mgy = std::max(1, p->desc.n_planes);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)p->persist_ctas);
+    cfg.blockDim = dim3(k2dThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    // The barrier words start every launch at zero: a launch that timed out leaves its arrival count behind.
+    TFD_CUDA(cudaMemsetAsync(p->arena + p->L.grid_bar, 0, 2 * sizeof(unsigned), s));
+    TFD_CUDA(cudaLaunchKernelEx(&cfg, k_step2d_persistent<T>, (const Grid<T> *)(p->arena + p->L.grid_tab),
+                                (const Tile2D *)(p->arena + p->L.tile_tab), p->tile2d_interior, p->L.tiles2d, m, mgx, mgy, nsteps,
+                                p->ptr<unsigned>(p->L.grid_bar)));
+    return TFD_OK;
+}
+
 // One two-pass step: the E pass, the dispersive samples, the TFSF boxes' E half step and E corrections, the H pass, the H half step and H
 // corrections. Unless the H pass ends the step, the observation launch (step_t) or k_pass_advance follows.
 template <typename T>
@@ -1915,6 +1967,7 @@ int step_t(tfd_plan *p, int nsteps, cudaStream_t s) {
         if (nsteps > 0) TFD_CHECK(launch_cluster2d<T>(p, nsteps, s));
         return TFD_OK;
     }
+    if (p->kernel == TFD_KERNEL_TILE2D && p->persist_ctas > 0 && nsteps >= kPassMany) return launch_persist2d<T>(p, nsteps, s);
     const PassShape &shape = nsteps < kPassMany ? p->pass_few : p->pass_many;
     if (p->two_pass && shape.ctas > 0) return launch_pass_steps<T>(p, shape, p->pass<T>(), nsteps, true, s);
     const int end = p->two_pass && pass_ends_step<T>(p);
@@ -2256,6 +2309,10 @@ int tfd_kernel_in_use(const tfd_plan *p, int32_t *kernel) {
 int tfd_step_launches(const tfd_plan *p, int32_t nsteps, int64_t *launches) {
     if (!p || !launches) return fail(TFD_ERR_INVALID, "null argument");
     if (nsteps < 0) return fail(TFD_ERR_INVALID, "nsteps must be non-negative");
+    if (p->persist_ctas > 0 && nsteps >= kPassMany && !p->in_batch) {
+        *launches = 1;
+        return TFD_OK;
+    }
     if (p->two_pass && (nsteps < kPassMany ? p->pass_few : p->pass_many).ctas > 0) {
         *launches = ((int64_t)nsteps + kPassLaunchSteps - 1) / kPassLaunchSteps;
         return TFD_OK;

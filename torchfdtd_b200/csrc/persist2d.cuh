@@ -1,4 +1,4 @@
-// Persistent stepping of a batch of 2D TMz grids: one cooperative launch runs many steps. Every warp walks the batch's strip
+// Persistent stepping of a 2D TMz grid, or a batch of them: one cooperative launch runs many steps. Every warp walks the strip
 // table (interior strips on the lean path, the rest on the general path, as the per-step kernels do), a grid-wide barrier
 // separates the steps, and the observations of step n - 1 (traces, DFT planes) are taken while step n computes: they read
 // the parity step n - 1 wrote, step n writes the other one, and they finish before the barrier after step n, that is
@@ -52,6 +52,49 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, int *status) {
     }
     __syncthreads();
     return ok != 0;
+}
+
+// Observations of step n, spread over the launch's blocks as the per-step observation kernel spreads them
+// over its (mgx x mgy) grid.
+template <typename T>
+__device__ __forceinline__ void observe_step(const MonitorArgs<T> &m, int mgx, int mgy, long long n) {
+    for (int b = blockIdx.x; b < mgx * mgy; b += gridDim.x) monitor_work(m, b % mgx, b / mgx, n, mgx);
+}
+
+// `count` steps of one 2D TMz plan: strips [0, interior) take the lean path, [interior, all) the general
+// one; warps are strided over the table. bar: the plan's barrier words (the launcher zeroes them before
+// every launch, so a launch that timed out leaves no stale arrival count to the next one).
+template <typename T>
+__global__ void __launch_bounds__(k2dThreads, 2) k_step2d_persistent(const Grid<T> *__restrict__ grids,
+                                                                    const Tile2D *__restrict__ strips, int interior, int all,
+                                                                    const __grid_constant__ MonitorArgs<T> m, int mgx, int mgy,
+                                                                    int count, unsigned *bar) {
+    const Grid<T> &g = grids[0];
+    const long long n0 = *m.counter;
+    const int lane = threadIdx.x & 31;
+    const int warps_total = gridDim.x * k2dWarps;
+    const int w0 = blockIdx.x * k2dWarps + (threadIdx.x >> 5);
+    long long n = n0;
+    for (int k = 0; k < count && n < m.steps; ++k, ++n) {
+        const int par = (int)(n & 1);
+        if (k > 0) observe_step(m, mgx, mgy, n - 1);
+        for (int s = w0; s < all; s += warps_total) {
+            const Tile2D st = strips[s];
+            if (s < interior) {
+                // The lean path reads x0-1, x0+31, y0-1 and y1 unchecked: refuse a strip that is not interior.
+                if (st.kind != 1 || st.x0 < 1 || st.x0 + 31 > g.n[0] - 1 || st.y0 < 1 || st.y1 > g.n[1] - 1 || st.y1 < st.y0) {
+                    if (lane == 0) atomicExch(g.status, kStatusBadStrip);
+                    continue;
+                }
+                strip_interior(g, st, par, lane);
+            } else {
+                strip_general(g, st, n, par, lane);
+            }
+        }
+        if (!grid_barrier(bar, g.status)) return;
+    }
+    if (n > n0) observe_step(m, mgx, mgy, n - 1);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *m.counter = n;
 }
 
 // `count` steps of a batch of 2D TMz plans of any sizes in one cooperative launch: the batch's strip table
