@@ -254,3 +254,27 @@ def test_calls_of_any_length_match_the_oracle(shape, precision, plane):
         assert np.linalg.norm(grid.get_plane(k) - value) <= 1e-12 * np.linalg.norm(value) and np.linalg.norm(value) > 0
     assert grid.counter() == plan.steps and grid.device_status() == 0
     grid.close()
+
+
+def test_pole_states_do_not_depend_on_the_order_of_the_samples():
+    """The library numbers a state's samples in memory order: any order of the caller's gives the same run, a sample listed
+    twice or by two states is refused."""
+    from torchfdtd_b200.native import NativeGrid
+    plan = plan_grid(dispersive(scene((21, 22, 23), 'float32')))
+    state = plan.ade[0]
+    assert len(plan.ade) == 1 and state.samples > 100
+    order = np.random.default_rng(2).permutation(state.samples)
+    half = state.samples // 2
+    out = []
+    for ade in ([state], [replace(state, target=state.target[order])], [replace(state, target=state.target[half:]), replace(state, target=state.target[:half])]):
+        grid = NativeGrid(replace(plan, ade=ade))
+        grid.step(plan.steps)
+        out.append((*grid.get_fields(), np.array(grid.diagnose())))
+        grid.close()
+    for other in out[1:]:
+        for a, b in zip(out[0][:2], other[:2]):
+            np.testing.assert_array_equal(a, b)
+        np.testing.assert_allclose(other[2], out[0][2], rtol=1e-12)
+    for ade in ([replace(state, target=np.append(state.target[:-1], state.target[0]))], [state, replace(state, target=state.target[5:6])]):
+        with pytest.raises(ValueError, match='overlap'):
+            NativeGrid(replace(plan, ade=ade))

@@ -715,22 +715,46 @@ int create_typed(tfd_plan *p, const tfd_desc *d, cudaStream_t s) {
     g.ade_at = nullptr;
     g.ade_samples = 0;
     if (d->n_ade > 0) {
-        std::vector<int> map((size_t)3 * L.count, -1);
+        // The samples of each state are numbered in memory order (component, z, y, x): consecutive cells of a row hold
+        // consecutive pole states (the caller's order, z fastest, scattered a row's states over 32-byte sectors). A sample's
+        // number is the count of its state's elements before it, from a bit per element.
+        const size_t words = ((size_t)3 * L.count + 63) / 64;
+        std::vector<uint64_t> taken(words, 0), bits(words);
+        std::vector<int> before(words);
+        std::vector<long long> at, element;
         int start = 0;
         for (int k = 0; k < d->n_ade; ++k) {
             const tfd_ade &m = d->ade[k];
             AdeDev<T> &st = g.ade[k];
             st.start = start;
             st.samples = m.samples;
+            std::fill(bits.begin(), bits.end(), 0);
+            element.resize(m.samples);
             st.poles = m.poles;
             for (int j = 0; j < m.samples; ++j) {
                 const long long cell = m.target[j] / 3;
                 const int comp = (int)(m.target[j] % 3);
                 const int x = (int)(cell / ((long long)n[1] * n[2])), y = (int)((cell / n[2]) % n[1]), z = (int)(cell % n[2]);
-                int &slot = map[(size_t)comp * L.count + (size_t)z * g.plane + (size_t)y * L.pitch + x];
-                if (slot >= 0) return fail(TFD_ERR_INVALID, "dispersive material states overlap");
-                slot = start + j;
+                const size_t e = (size_t)comp * L.count + (size_t)z * g.plane + (size_t)y * L.pitch + x;
+                if ((taken[e >> 6] >> (e & 63)) & 1) return fail(TFD_ERR_INVALID, "dispersive material states overlap");
+                taken[e >> 6] |= 1ull << (e & 63);
+                bits[e >> 6] |= 1ull << (e & 63);
+                element[j] = (long long)e;
             }
+            int count = 0;
+            for (size_t q = 0; q < words; ++q) {
+                before[q] = count;
+                count += __builtin_popcountll(bits[q]);
+            }
+            std::vector<double> weight(L.ade[k].weight ? m.samples : 0);
+            at.resize((size_t)start + m.samples);
+            for (int j = 0; j < m.samples; ++j) {
+                const size_t e = (size_t)element[j];
+                const int to = before[e >> 6] + __builtin_popcountll(bits[e >> 6] & ((1ull << (e & 63)) - 1));
+                at[(size_t)start + to] = (long long)e;
+                if (L.ade[k].weight) weight[to] = m.weight[j];
+            }
+            if (int rc = upload(s, p, L.ade[k].weight, weight)) return rc;
             start += m.samples;
             std::vector<T> coef((size_t)3 * m.poles);
             T ksum = T(0);
@@ -752,25 +776,6 @@ int create_typed(tfd_plan *p, const tfd_desc *d, cudaStream_t s) {
             st.P = p->ptr<T>(L.ade[k].state);
             st.Q = st.P + (size_t)m.poles * m.samples;
         }
-        // Renumber the samples of each state in memory order (component, z, y, x): consecutive cells of a row hold
-        // consecutive pole states. The caller's order (z fastest) scattered a row's states over 32-byte sectors.
-        std::vector<int> renumbered(start), next(d->n_ade, 0);
-        std::vector<long long> at(start);
-        for (size_t e = 0; e < map.size(); ++e) {
-            if (map[e] < 0) continue;
-            int k = 0;
-            while (k + 1 < d->n_ade && map[e] >= g.ade[k + 1].start) ++k;
-            const int to = g.ade[k].start + next[k]++;
-            renumbered[map[e]] = to;
-            map[e] = to;
-            at[to] = (long long)e;
-        }
-        for (int k = 0; k < d->n_ade; ++k)
-            if (L.ade[k].weight) {
-                std::vector<double> w(d->ade[k].samples);
-                for (int j = 0; j < d->ade[k].samples; ++j) w[renumbered[g.ade[k].start + j] - g.ade[k].start] = d->ade[k].weight[j];
-                if (int rc = upload(s, p, L.ade[k].weight, w)) return rc;
-            }
         // The sample map is read only where a soft E source drives a dispersive sample.
         bool driven = false;
         for (int t = 0; t < d->n_sources && !driven; ++t) {
@@ -778,13 +783,17 @@ int create_typed(tfd_plan *p, const tfd_desc *d, cudaStream_t s) {
             if (q.family != 0) continue;
             for (int z = q.lo[2]; z < q.hi[2] && !driven; ++z)
                 for (int y = q.lo[1]; y < q.hi[1] && !driven; ++y)
-                    for (int x = q.lo[0]; x < q.hi[0] && !driven; ++x)
-                        driven = map[(size_t)q.component * L.count + (size_t)z * g.plane + (size_t)y * L.pitch + x] >= 0;
+                    for (int x = q.lo[0]; x < q.hi[0] && !driven; ++x) {
+                        const size_t e = (size_t)q.component * L.count + (size_t)z * g.plane + (size_t)y * L.pitch + x;
+                        driven = (taken[e >> 6] >> (e & 63)) & 1;
+                    }
         }
         if (int rc = upload(s, p, L.ade_at, at)) return rc;
         g.ade_at = p->ptr<long long>(L.ade_at);
         g.ade_samples = start;
         if (driven) {
+            std::vector<int> map((size_t)3 * L.count, -1);
+            for (int j = 0; j < start; ++j) map[at[j]] = j;
             if (int rc = upload(s, p, L.ade_map, map)) return rc;
             for (int c = 0; c < 3; ++c) g.ade_map[c] = p->ptr<int>(L.ade_map) + (size_t)c * L.count;
         }
