@@ -154,6 +154,17 @@ __device__ __forceinline__ void pass_cpml(const PassArgs<T> &A, const PassCell<I
     if (snap != nullptr) pack_store(snap + p, m);
 }
 
+// The cell of an element index of a component array. A plane of a 2D grid may hold 2^31 elements and more.
+struct CellAt { int x, y, z; };
+__host__ __device__ constexpr CellAt cell_at(long long i, long long plane, int pitch) {
+    const long long rest = i % plane;
+    const int z = (int)(i / plane);
+    if (rest < (1LL << 31)) return CellAt{(int)rest % pitch, (int)rest / pitch, z};       // a fraction of the 64-bit division
+    return CellAt{(int)(rest % pitch), (int)(rest / pitch), z};
+}
+static_assert(cell_at(65000LL * 65536 + 7, 65536LL * 65536, 65536).y == 65000 && cell_at(65000LL * 65536 + 7, 65536LL * 65536, 65536).x == 7,
+              "element indices of large planes");
+
 // Dispersive samples (threads j of total): the coupled trapezoidal ADE turns the free update that the E pass stored into
 // E_new and advances the pole states, then the soft sources of the cell are added (the E pass leaves dispersive samples
 // to this sweep). Reference operation order (torchfdtd/materials.py:67-88).
@@ -191,10 +202,11 @@ __device__ __forceinline__ void pass_ade(const Grid<T> &g, int j, int par, long 
         }
     }
     if (g.n_src > 0) {
-        const int z = (int)(i / g.plane), y = (int)(i % g.plane) / g.pitch, x = (int)(i % g.plane) % g.pitch;
+        const CellAt cell = cell_at(i, g.plane, g.pitch);
         for (int t = 0; t < g.n_src; ++t) {
             const SourceTerm &q = g.src[t];
-            if (q.family == 0 && q.comp == c && x >= q.lo[0] && x < q.hi[0] && y >= q.lo[1] && y < q.hi[1] && z >= q.lo[2] && z < q.hi[2])
+            if (q.family == 0 && q.comp == c && cell.x >= q.lo[0] && cell.x < q.hi[0] && cell.y >= q.lo[1] && cell.y < q.hi[1] &&
+                cell.z >= q.lo[2] && cell.z < q.hi[2])
                 e = e + g.src_values[(long long)t * g.steps + n];
         }
     }
