@@ -147,9 +147,9 @@ def test_plane_fields_match_the_forward_simulation_planes():
 
 
 @pytest.mark.parametrize('precision', ['float32', 'float64'])
-def test_interior_tiles_fast_path_is_the_general_path(monkeypatch, precision):
-    """A grid with whole interior tiles (80 x 40 x 30 cells, CPML 6): the reverse-step kernels' interior fast path
-    gives the general path's gradient bitwise, and (FP64) the oracle's."""
+def test_plain_rows_of_the_reverse_step_match_the_oracle(precision):
+    """A grid whose reverse step has plain rows (80 x 40 x 30 cells, CPML 6: no face or slab near them) beside the others: the
+    oracle's gradient, relative L2 1e-5 in FP32 (sums of 30 steps' products in another order) and 1e-11 in FP64."""
     import torch
     from torchfdtd_b200.adjoint import DifferentiableSimulation
     from torchfdtd_b200.models import Monitor, Source
@@ -161,18 +161,13 @@ def test_interior_tiles_fast_path_is_the_general_path(monkeypatch, precision):
     dtype = torch.float32 if precision == 'float32' else torch.float64
     eps = np.random.default_rng(5).uniform(1, 3, size=plan.shape)
     w = np.random.default_rng(6).normal(size=(plan.steps, 2))
-    grads = {}
-    for fast in ('1', '0'):
-        monkeypatch.setenv('TFD_ADJ_FAST', fast)
-        model = DifferentiableSimulation(project)
-        epsilon = torch.tensor(eps, dtype=dtype, device='cuda', requires_grad=True)
-        result = model(epsilon)
-        (result.signals * torch.tensor(w, dtype=dtype, device='cuda')).sum().backward()
-        grads[fast] = epsilon.grad.cpu().numpy()
-        model.close()
-    np.testing.assert_array_equal(grads['1'], grads['0'])
-    assert np.abs(grads['1']).max() > 0
-    if precision == 'float64':
-        oracle = AdjointOracle(plan, eps)
-        oracle.forward()
-        assert rel(grads['1'], oracle.backward(w)) <= 1e-11
+    model = DifferentiableSimulation(project)
+    epsilon = torch.tensor(eps, dtype=dtype, device='cuda', requires_grad=True)
+    result = model(epsilon)
+    (result.signals * torch.tensor(w, dtype=dtype, device='cuda')).sum().backward()
+    grad = epsilon.grad.cpu().numpy()
+    model.close()
+    oracle = AdjointOracle(plan, eps.astype(plan.dtype))
+    oracle.forward()
+    assert np.abs(grad).max() > 0
+    assert rel(grad, oracle.backward(w.astype(plan.dtype))) <= (1e-5 if precision == 'float32' else 1e-11)

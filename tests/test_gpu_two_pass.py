@@ -1,5 +1,5 @@
-"""The two-pass step kernels and the reverse step's two passes against the NumPy oracle: every way they are launched (three launches per step, one cluster,
-one cooperative launch), at row lengths around the 16-byte groups, and with more than two CPML slabs on an axis (the
+"""The two-pass step kernels and the reverse step's two passes against the NumPy oracle: every way they are launched (launches
+per pass, one cluster, one cooperative launch), at row lengths around the 16-byte groups, and with more than two CPML slabs on an axis (the
 row-table path). Bars: fields, CPML memories and traces bitwise, like the other step kernels (same operations, same
 order, no contraction); gradients within the relative L2 of tests/test_gpu_adjoint.py."""
 from dataclasses import replace
@@ -26,7 +26,7 @@ def scene(shape, precision, faces=None, component='Ey', steps=12):
                    monitors=[Monitor(center=(-.1, .05, 0), component=component)])
 
 
-def assert_matches_oracle(plan, seed, kernel='gather'):
+def assert_matches_oracle(plan, seed, kernel='gather', launches=None):
     from torchfdtd_b200.native import NativeGrid
     rng = np.random.default_rng(seed)
     oracle = YeeOracle(plan)
@@ -36,6 +36,7 @@ def assert_matches_oracle(plan, seed, kernel='gather'):
             if family + 'xyz'[c] in advanced:
                 field[..., c] = rng.normal(size=plan.shape).astype(plan.dtype)
     grid = NativeGrid(plan, kernel=kernel)
+    assert launches is None or grid.step_launches(5) == launches
     grid.set_fields(oracle.E, oracle.H)
     grid.step(5)
     grid.step(plan.steps - 5)
@@ -59,7 +60,7 @@ PERIODIC_Y = {'y_min': BoundaryFace(kind='periodic'), 'y_max': BoundaryFace(kind
     ((32, 13, 14), 'float32', PERIODIC_Y, 'Ez'), ((65, 33, 1), 'float32', PERIODIC_Y, 'Hz'), ((67, 40, 1), 'float64', None, 'Ex')])
 def test_every_launch_form_matches_the_oracle(monkeypatch, mode, shape, precision, faces, component):
     monkeypatch.setenv('TFD_PASS_STEPS', mode)
-    assert_matches_oracle(plan_grid(scene(shape, precision, faces, component)), 3)
+    assert_matches_oracle(plan_grid(scene(shape, precision, faces, component)), 3, launches=10 if mode == '0' else 1)
 
 
 @pytest.mark.parametrize('precision', ['float32', 'float64'])
@@ -266,7 +267,8 @@ def test_pole_states_do_not_depend_on_the_order_of_the_samples():
     order = np.random.default_rng(2).permutation(state.samples)
     half = state.samples // 2
     out = []
-    for ade in ([state], [replace(state, target=state.target[order])], [replace(state, target=state.target[half:]), replace(state, target=state.target[:half])]):
+    halves = [replace(state, target=state.target[half:]), replace(state, target=state.target[:half])]
+    for ade in ([state], [replace(state, target=state.target[order])], halves):
         grid = NativeGrid(replace(plan, ade=ade))
         grid.step(plan.steps)
         out.append((*grid.get_fields(), np.array(grid.diagnose())))
@@ -278,3 +280,68 @@ def test_pole_states_do_not_depend_on_the_order_of_the_samples():
     for ade in ([replace(state, target=np.append(state.target[:-1], state.target[0]))], [state, replace(state, target=state.target[5:6])]):
         with pytest.raises(ValueError, match='overlap'):
             NativeGrid(replace(plan, ade=ade))
+
+
+@pytest.mark.parametrize('mode,launches', [('0', 15), ('2', 1)])
+@pytest.mark.parametrize('precision', ['float32', 'float64'])
+def test_dispersive_sweep_matches_the_oracle(monkeypatch, precision, mode, launches):
+    """The sweep over the dispersive samples as a launch of its own (the form of every large plan) and inside the one launch; the
+    source drives some of the samples."""
+    monkeypatch.setenv('TFD_PASS_STEPS', mode)
+    assert_matches_oracle(plan_grid(dispersive(scene((21, 22, 23), precision))), 6, launches=launches)
+
+
+@pytest.mark.parametrize('shape,precision,component,metal', [
+    ((13, 14, 15), 'float32', 'Ey', False), ((14, 13, 16), 'float64', 'Hz', False), ((65, 33, 1), 'float32', 'Hz', False),
+    ((21, 22, 23), 'float32', 'Ey', True)])
+def test_64_bit_index_variant_matches_the_oracle(monkeypatch, shape, precision, component, metal):
+    """The kernels of arrays of 2^31 elements and more, at a size that a test can hold."""
+    monkeypatch.setenv('TFD_PASS_WIDE', '1')
+    project = scene(shape, precision, component=component)
+    assert_matches_oracle(plan_grid(dispersive(project) if metal else project), 7, launches=15 if metal else 10)
+
+
+def test_planes_past_65535_match_the_oracle(monkeypatch):
+    """A pass walks the planes that its launch grid cannot number."""
+    from oracle.cpu import CpuOracle
+    from torchfdtd_b200.native import NativeGrid
+    monkeypatch.setenv('TFD_PASS_STEPS', '0')
+    project = scene((13, 13, 65700), 'float32', steps=10)
+    project.sources[0].center = (.1, 0, 1635.0)
+    plan = plan_grid(project)
+    assert plan.shape == (13, 13, 65700)
+    grid = NativeGrid(plan, kernel='gather')
+    rng = np.random.default_rng(4)
+    oracle = CpuOracle(plan)
+    oracle.E[:] = rng.normal(size=oracle.E.shape).astype(np.float32)
+    grid.set_fields(oracle.E, oracle.H)
+    grid.step(4)
+    oracle.run(4)
+    E, H = grid.get_fields()
+    np.testing.assert_array_equal(E, oracle.E)
+    np.testing.assert_array_equal(H, oracle.H)
+    grid.close()
+
+
+@pytest.mark.parametrize('wide', [False, True])
+@pytest.mark.parametrize('precision', ['float32', 'float64'])
+def test_reverse_step_variants_match_the_oracle(monkeypatch, precision, wide):
+    """A grid with plain rows, rows near a face or slab and groups near an x slab: each variant of the reverse step's passes."""
+    import torch
+    from torchfdtd_b200.adjoint import DifferentiableSimulation
+    if wide:
+        monkeypatch.setenv('TFD_PASS_WIDE', '1')
+    project = scene((40, 24, 22), precision, steps=20)
+    plan = plan_grid(project)
+    rng = np.random.default_rng(12)
+    eps, w = rng.uniform(1, 3, size=plan.shape), rng.normal(size=(plan.steps, 1))
+    dtype = torch.float32 if precision == 'float32' else torch.float64
+    model = DifferentiableSimulation(project)
+    epsilon = torch.tensor(eps, dtype=dtype, device='cuda', requires_grad=True)
+    (model(epsilon).signals * torch.tensor(w, dtype=dtype, device='cuda')).sum().backward()
+    oracle = AdjointOracle(plan, eps.astype(plan.dtype))
+    oracle.forward()
+    want = oracle.backward(w.astype(plan.dtype))
+    assert np.linalg.norm(epsilon.grad.cpu().numpy() - want) <= (1e-5 if precision == 'float32' else 1e-11) * np.linalg.norm(want)
+    assert np.linalg.norm(want) > 0
+    model.close()

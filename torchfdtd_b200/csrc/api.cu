@@ -1762,6 +1762,7 @@ int setup_pass(tfd_plan *p) {
     for (int f = 0; f < 2; ++f) a.split[f] = pass_split<T>(p, f, 0);
     a.magic_total = pass_magic(a.split[0].total);
     p->pass_metric = false;
+    p->pass_wide = getenv("TFD_PASS_WIDE") != nullptr;    // the variant of the largest grids at any size, for comparisons
     for (int f = 0; f < 2; ++f)
         for (int ax = 0; ax < 3; ++ax) {
             p->pass_metric = p->pass_metric || a.g.metric[f][ax] != nullptr;
