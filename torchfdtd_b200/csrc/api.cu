@@ -349,13 +349,15 @@ int strip_capacity(int nx, int ny) { return ((nx + k2dOwnX - 1) / k2dOwnX) * ((n
 //   line lies at kPassGridGroups64: 128^3: 86.9 / 92.3; 140^3: 106 / 118;
 // - launches where the samples of the planes outnumber the cooperative form's threads: 160 x 120 x 40 cells with 147,408 samples of
 //   20 frequencies: 57.1 / 50.3; with 17,472 of 200: 74 / 79.
-// Calls of fewer than kPassMany steps (a captured single step is how Simulation.run replays) do not earn the cooperative launch's
-// 5-7 us back: 60^3 cells, one step: 22.6 against 21.3; TE, 350 x 300: 14.5 / 12.5. The cluster's does not cost them: TE, 200 x 121: 10.4 /
-// 11.4, while its observations are light (630 samples of 20 frequencies: 16.4 / 18.6; of 200: 39.1 / 33).
+// Calls of fewer than kPassMany steps (a captured single step is how Simulation.run replays) earn the cooperative launch's 5-7 us
+// back only on larger grids with x slabs: 60^3 cells, one step: 22.6 against 21.3 in launches; 80^3: 22.3 / 25.7; 100^3: 36.3 / 39; FP64, 60^3:
+// 24.4 / 22.8; 100^3: 57.2 / 61.9; periodic 100^3: 24.8 / 21.8; TE, 350 x 300: 14.5 / 12.5. The cluster's does not cost them: TE, 200 x 121:
+// 10.4 / 11.4, while its observations are light (630 samples of 20 frequencies: 16.4 / 18.6; of 200: 39.1 / 33).
 constexpr int kPassClusterRanks = 16;
 constexpr long long kPassClusterGroups = (long long)kPassClusterRanks * kPassStepThreads, kPassFewSweeps = 6;
 constexpr long long kPassGridGroups = kPassFewSweeps * 148 * kPassStepThreads, kPassGridGroups64 = 3LL << 19;
 constexpr long long kPassLightSums = 1LL << 15;           // accumulators
+constexpr long long kPassFewCost = 5LL << 15;             // groups, those that meet an x slab three times
 constexpr int kPassMany = 4;
 
 // Steps of one launch at most: the barrier counts every arrival of a launch in 32 bits, three per step and CTA (two without
@@ -1598,20 +1600,38 @@ PassSteps<T> pass_steps_kernel(tfd_plan *p, bool cluster) {
 }
 
 constexpr long long kMarchMinCells = 1LL << 26;      // see two_pass_3d
-// A plane's chunks end with its x-slab groups, the slow ones. Moved on by `rotate` CTAs from sweep to sweep, a CTA's chunks
-// lie 1 / sweeps of a plane apart, so that all CTAs meet slab groups about equally often: 100^3 cells 33.7 -> 30.0 us per step,
-// 110^3 40.0 -> 32.6, 120^3 47.9 -> 40.9. Over many sweeps the chunks mix by themselves (FP64, 140^3: 105 us, 111 when rotated).
-unsigned pass_steps_rotation(long long total, long long groups, int ctas, int threads) {
-    const double chunks = (double)total / threads;
-    const long long sweeps = (groups + (long long)ctas * threads - 1) / ((long long)ctas * threads);
-    if (sweeps < 2 || sweeps > kPassFewSweeps || chunks <= 1) return 0;
-    unsigned best = 0;
-    double least = 1;
-    for (int r = 0; r < ctas && r <= 2 * chunks; ++r) {
-        const double turns = (ctas + r) / chunks, off = std::fabs(turns - std::floor(turns) - 1.0 / sweeps);
-        if (off < least) { least = off; best = r; }
+// A plane's chunks end with its x-slab groups, which cost about three plain ones. CTAs that meet them in every sweep hold up the
+// barrier, so the chunks move on by `rotate` CTAs from sweep to sweep: the rotation under which the busiest CTA has least to do.
+// us per step, not rotated / rotated: 70 x 200 x 80 cells (CPML 8): 48.4 / 35.8; 110^3 (CPML 10): 50.5 / 41.1; 90 x 140 x 110 (CPML 14):
+// 52.4 / 43.7; 120 x 90 x 60 (CPML 8): 28.0 / 21.0. Over many sweeps the chunks mix by themselves.
+unsigned pass_steps_rotation(const PassSplit &split, long long groups, int ctas, int threads) {
+    const int chunks = (int)((groups + threads - 1) / threads), sweeps = (chunks + ctas - 1) / ctas;
+    if (sweeps < 2 || sweeps > kPassFewSweeps) return 0;
+    const long long total = split.total, plain = split.plain_total;
+    auto slabs_before = [&](long long i) { return i / total * (total - plain) + std::max<long long>(0, i % total - plain); };
+    std::vector<long long> cost(chunks);
+    for (int k = 0; k < chunks; ++k) {
+        const long long a = (long long)k * threads, b = std::min(groups, a + threads);
+        cost[k] = b - a + 2 * (slabs_before(b) - slabs_before(a));
     }
-    return best;
+    int best = 0;
+    double least = -1, least_squares = 0;                 // equal maxima: the more even rotation
+    for (int r = 0; r < ctas; ++r) {
+        double most = 0, squares = 0;
+        for (int c = 0; c < ctas; ++c) {
+            long long sum = 0;
+            for (int k = 0, at = c; k < sweeps; ++k, at = (at + r) % ctas)
+                if (k * ctas + at < chunks) sum += cost[k * ctas + at];
+            most = std::max(most, (double)sum);
+            squares += (double)sum * (double)sum;
+        }
+        if (least < 0 || most < least || (most == least && squares < least_squares)) {
+            least = most;
+            least_squares = squares;
+            best = r;
+        }
+    }
+    return (unsigned)best;
 }
 
 inline void pass_steps_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &attr, const PassShape &shape, cudaStream_t s) {
@@ -1675,7 +1695,7 @@ int setup_pass_steps(tfd_plan *p) {
         const long long want = (groups + grid.threads - 1) / grid.threads + mblocks;
         if (per_sm > 0) grid.ctas = (int)std::min<long long>(want, ctas);
         grid.chunks = (unsigned)((groups + grid.threads - 1) / grid.threads);
-        grid.rotate = pass_steps_rotation(a.split[0].total, groups, grid.ctas, grid.threads);
+        grid.rotate = pass_steps_rotation(a.split[0], groups, grid.ctas, grid.threads);
     }
     if (mode >= 0) {
         p->pass_many = p->pass_few = mode == 1 ? cluster : grid;
@@ -1683,7 +1703,9 @@ int setup_pass_steps(tfd_plan *p) {
     }
     if (samples == 0) p->pass_many = cluster.ctas > 0 ? cluster : grid;
     else if (samples <= (long long)grid.ctas * grid.threads) p->pass_many = grid;
-    if (sums <= kPassLightSums) p->pass_few = cluster;
+    if (cluster.ctas > 0 && sums <= kPassLightSums) p->pass_few = cluster;
+    const long long slab = (long long)(a.split[0].total - a.split[0].plain_total) * a.g.n[2];
+    if (cluster.ctas == 0 && slab > 0 && groups + 2 * slab >= kPassFewCost) p->pass_few = p->pass_many;
     return TFD_OK;
 }
 
