@@ -345,3 +345,19 @@ def test_reverse_step_variants_match_the_oracle(monkeypatch, precision, wide):
     assert np.linalg.norm(epsilon.grad.cpu().numpy() - want) <= (1e-5 if precision == 'float32' else 1e-11) * np.linalg.norm(want)
     assert np.linalg.norm(want) > 0
     model.close()
+
+
+@pytest.mark.parametrize('shape,sampling,kernel', [((512, 512, 128), 'cell', 'march'), ((256, 256, 512), 'cell', 'gather'),
+                                                   ((512, 512, 126), 'cell', 'gather'), ((512, 512, 128), 'yee', 'gather')])
+def test_default_kernel_of_large_uniform_grids(shape, sampling, kernel):
+    """The marching kernel from 2^25 cells on where the grid fills its tiles; the bitwise equality of both at such a size is
+    tests/test_gpu_configs.py's."""
+    import torch
+    from torchfdtd_b200.native import NativeGrid
+    project = scene(shape, 'float32')
+    project.region.material_sampling = sampling
+    plan = plan_grid(project, material=False)
+    plan.epsilon, plan.inv_eps = torch.ones(plan.shape if sampling == 'cell' else (*plan.shape, 3), device='cuda'), None
+    grid = NativeGrid(plan, material=plan.epsilon)
+    assert grid.kernel == kernel
+    grid.close()

@@ -1599,7 +1599,6 @@ PassSteps<T> pass_steps_kernel(tfd_plan *p, bool cluster) {
     }
 }
 
-constexpr long long kMarchMinCells = 1LL << 26;      // see two_pass_3d
 // A plane's chunks end with its x-slab groups, which cost about three plain ones. CTAs that meet them in every sweep hold up the
 // barrier, so the chunks move on by `rotate` CTAs from sweep to sweep: the rotation under which the busiest CTA has least to do.
 // us per step, not rotated / rotated: 70 x 200 x 80 cells (CPML 8): 48.4 / 35.8; 110^3 (CPML 10): 50.5 / 41.1; 90 x 140 x 110 (CPML 14):
@@ -1731,17 +1730,27 @@ int launch_pass_steps(tfd_plan *p, const PassShape &shape, const PassArgs<T> &a,
     return TFD_OK;
 }
 
-// Whether a 3D plan steps in two passes instead of the marching kernel. The marching kernel moves 52 bytes per cell
-// against 76, but needs the largest grids to get there; measured, us per step (two-pass / march): 160 x 120 x 40: 27 /
-// 43; 192^3: 136 / 207; 256^3: 281 / 398; 320^3: 514 / 647; 400^3: 971 / 1018; 512 x 512 x 256: 960-990 / 907. With
-// periodic x / y faces (512 x 512 x 128: 465 / 626), a nonuniform mesh (306 x 306 x 176: 314 / 379) or in FP64 (151 x 133 x
-// 117, periodic: 89 / 222) the marching kernel runs slower bodies and the two passes win at every size tried. Kernel
-// 'march' by name, an explicit launch variant or TFD_MARCH_VARIANT asks for the marching kernel.
+// Whether a 3D plan steps in two passes instead of the marching kernel, which moves 52 bytes per cell against 76 but computes
+// whole tiles of 31 x 15 cells and their halos. us per step (two passes / march, and the share of the tiles' cells that are the
+// grid's), uniform FP32, one permittivity per cell: 192^3: 133 / 178 (0.87); 256^3: 276 / 336 (0.87); 300 x 310 x 330 (31 M cells): 515 / 528 (0.95);
+// from 2^25 cells on: 512 x 512 x 128: 521 / 502 (0.95); 256 x 256 x 512: 531 / 621 (0.87); 350 x 300 x 320: 535 / 551 (0.94); 400 x 330 x 300: 614 /
+// 588 (0.99); 350^3: 668 / 702 (0.91); 400 x 400 x 300: 734 / 706 (0.98); 512 x 512 x 192: 751 / 702 (0.95); 500 x 500 x 300: 1118 / 1117 (0.93);
+// 512 x 512 x 256: 981 / 905; 448^3: 1300 / 1248 (0.96); 512^3: 1902 / 1717; 700 x 600 x 400: 2377 / 2294 (0.98). With three permittivities per
+// cell the two are even up to 2^27 cells (400^3: 1005 / 1025; 500 x 500 x 300: 1164 / 1249; 512^3: 1987 / 1960). The marching kernel's bodies
+// for periodic x / y faces (512 x 512 x 128: 464 / 569; 600 x 500 x 300: 1184 / 1340), nonuniform meshes (798 x 618 x 402: 3009 / 3160) and FP64 (400 x
+// 400 x 300: 1779 / 1797; 500 x 450 x 350: 2856 / 2958) were behind at every size measured, up to 198 M cells. Kernel 'march' by name, an
+// explicit launch variant or TFD_MARCH_VARIANT asks for the marching kernel.
+constexpr long long kMarchMinCells = 1LL << 25, kMarchMinCells3 = 1LL << 27;
+constexpr double kMarchMinFill = 0.945;
+
 bool two_pass_3d(const tfd_plan *p) {
     const tfd_desc &d = p->desc;
     if (d.kernel == TFD_KERNEL_MARCH || d.launch_variant != 0 || getenv("TFD_MARCH_VARIANT")) return false;
     const bool seams = d.face[0][0] == TFD_FACE_PERIODIC || d.face[1][0] == TFD_FACE_PERIODIC;
-    return d.precision == 8 || p->march_metric || seams || (long long)d.nx * d.ny * d.nz < kMarchMinCells;
+    if (d.precision == 8 || p->march_metric || seams) return true;
+    const long long tiles_x = (d.nx + 30) / 31, tiles_y = (d.ny + 14) / 15;
+    const double fill = (double)d.nx * d.ny / (double)(tiles_x * 31 * tiles_y * 15);
+    return (long long)d.nx * d.ny * d.nz < (d.material_samples == 3 ? kMarchMinCells3 : kMarchMinCells) || fill < kMarchMinFill;
 }
 
 // The multiplier that pass_divide takes for a division by d.
