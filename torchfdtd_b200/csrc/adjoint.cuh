@@ -1,4 +1,4 @@
-// Discrete adjoint of one Yee/CPML step, gather form: one thread per cell.
+// Discrete adjoint of one Yee/CPML step: two passes, one thread per 16-byte group of cells of a row.
 //
 // The forward step n maps the state s_n = (E, H, psi) to s_{n+1}:
 //     E' = E + (cn / eps) curl_b(H; psi_E)      then E sources
@@ -22,8 +22,8 @@
 // families' adjoint CPML memories are double-buffered by reverse-step parity; each memory is written once, by the thread
 // that owns its cell. The forward state comes from a snapshot of s_n, so no forward buffer is disturbed.
 //
-// What bounds them on large grids is DRAM: in FP32 60 bytes per cell in the E pass (h_bar, the snapshot's H, e_bar and S
-// read, e_bar and S written) and 40 in the H pass.
+// In FP32 they must move 72 bytes per cell in the E pass (h_bar, the snapshot's H, e_bar and S read, e_bar and S written) and 40
+// in the H pass (e_bar, 1/eps and h_bar read, h_bar written): 36 and 20 us at 200 x 200 x 80 cells and the copy rate.
 //
 // The material sensitivity is accumulated as S_c = sum_n e_bar_c * curl_b(H)_c per component; the host
 // forms dJ/d eps = -cn S / eps^2 (summed over components for a per-cell permittivity).
@@ -488,8 +488,9 @@ __device__ __forceinline__ bool adj_yz(const AdjArgs<T> &A, int y, int z) {
 }
 
 // Blocks per SM, us per launch at 200 x 200 x 80 cells, CPML 12, FP32: E pass 112 with two (128 registers), 123 with three;
-// H pass 75 with two, 60 with three. (One thread per cell: 180 and 100.) Both are far from the DRAM floor of 35 and 25 us: half
-// the rows meet a slab, whose terms triple the instructions, and the E pass holds 20 input vectors per thread.
+// H pass 75 with two, 60 with three. (One thread per cell: 180 and 100.) Both are far from the DRAM floor of 36 and 20 us (260
+// and 140 MB moved, CPML memories included): half the rows meet a slab, whose terms triple the instructions, and the E pass holds
+// 20 input vectors per thread.
 //
 // Blocks of kPassThreads groups of one plane (blockIdx.x; plain groups first, then those near an x slab), planes on
 // blockIdx.y: ascending in the E pass, descending in the H pass. Reads parity q, writes q^1.

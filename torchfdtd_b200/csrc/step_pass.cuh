@@ -8,10 +8,10 @@
 // Every input of a group is a load of its own, independent of the others: the H rows at y and y - 1, the planes z
 // and z - 1, E and 1/eps as 16-byte vectors, the x - 1 value as one scalar, all issued before the first use. What bounds
 // it on large grids is DRAM: 76 bytes per cell and step in FP32 (E pass: H, E, 1/eps read, E written; H pass: E, H read,
-// H written), 5.5 GB per step at 512 x 512 x 256 cells in 0.96-0.99 ms (5.6 TB/s, 87 % of the measured copy rate). The H
+// H written; 5.1 GB per step at 512 x 512 x 256 cells, and 0.4 GB of CPML memories) in 0.96-0.99 ms (5.5-5.7 TB/s, 86-88 % of the copy rate). The H
 // pass walks the planes in the opposite order of the E pass and starts on the E values that the E pass left in L2.
-// At 256^3 cells: 0.281 ms per step against 0.398 ms for the fused marching kernel (its halo recomputation and
-// per-row paths issue 11 warp-instructions per cell, these two passes 7) and 0.665 ms for one thread per cell with a
+// At 256^3 cells: 0.276-0.281 ms per step against 0.336 ms for the fused marching kernel (its halo recomputation and
+// per-row paths issue 11 warp-instructions per cell, these two passes 6.2) and 0.665 ms for one thread per cell with a
 // TFSF box. Not kept: the H pass trailing the E pass slab by slab in one launch, or in alternating launches, so that L2
 // serves the second reads (1.02-1.4 ms and 1.1-1.7 ms at 512 x 512 x 256: signalling and launch tails cost more than
 // the traffic saved).
