@@ -1807,8 +1807,9 @@ dim3 pass_blocks(const tfd_plan *p, unsigned total) {
 }
 
 // Whether the H pass ends the step (k_pass_h), point traces included: no planes, no boxes, few traces (one block records them)
-// and few blocks. us per captured step with a third launch / without: TE, 400 x 400 cells, 157 blocks: 10.5 / 8.9; 700 x 700, 480: 14.7 /
-// 13.7; 1000 x 1000, 977: 17.3 / 18.3; 60^3 cells, 240: 20.5 / 20.2; FP64 128^3, 4,096: 91 / 106.
+// and few blocks. us per captured step with a third launch / without: TE, 250 x 200 cells, 50 blocks: 12.2 / 11.4; 512 x 512, 256: 10.4 /
+// 9.3; 700 x 700, 479: 14.4 / 14.1; 850 x 850, 708: 15.6 / 15.6; 1000 x 1000, 977: 16.9 / 17.7; 60^3 cells, 240: 20.0 / 19.5; 80^3, 560: 23.3 / 23.7;
+// FP64 128^3, 4,096: 91 / 106.
 constexpr long long kPassEndBlocks = 512;
 constexpr int kPassEndTraces = 1024;
 

@@ -544,8 +544,8 @@ __global__ void __launch_bounds__(kPassThreads, kPassBlocks<T>) k_pass_e(const _
 }
 
 // end: nothing follows in the step but point traces, which the block that finishes last records before it advances the step
-// counter. A third launch costs 1-2 us on small grids (captured TE steps, 400 x 400 cells: 10.5 us with it, 8.9 without); with
-// many blocks their fences cost more than that (1000 x 1000: 17.3 and 18.3), see pass_ends_step in api.cu.
+// counter. A third launch costs about 1 us on small grids (captured TE steps, 400 x 400 cells: 10.8 us with it, 9.8 without; single
+// steps 12.5 and 11.7); with many blocks their fences cost more than that (1000 x 1000: 16.9 and 17.7), see pass_ends_step in api.cu.
 template <typename T, int ACTIVE, bool METRIC, typename I>
 __global__ void __launch_bounds__(kPassThreads, kPassBlocks<T>) k_pass_h(const __grid_constant__ PassArgs<T> A,
                                                                         const __grid_constant__ MonitorArgs<T> m, int end) {
